@@ -79,20 +79,6 @@ __device__ __forceinline__ void load_task(const CorrArgs &a, int ch, int ant, in
       w[q] = (ok_ant && p < a.npkt) ? __ldg(reinterpret_cast<const uint32_t *>(base + p * pstride))
                                     : 0u;
     }
-  } else if (FMT == FMT_REORDERED) {
-    // [pkt][2*nchan][64][2 pol] packed (the massage() output).
-    const int64_t pstride = (int64_t)2 * a.nchan * 64 * 2;
-    const uint8_t *base = a.in + ((int64_t)(2 * ch) * 64 + ant) * 2;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int p = p0 + q;
-      uint32_t lo = 0, hi = 0;
-      if (p < a.npkt) {
-        lo = __ldg(reinterpret_cast<const uint16_t *>(base + p * pstride));
-        hi = __ldg(reinterpret_cast<const uint16_t *>(base + p * pstride + 128));
-      }
-      w[q] = lo | (hi << 16);
-    }
   } else {
     // FMT_XGPU_INT8: [pkt][nfreq][64][2 pol][re, im] int8 (xGPU ComplexInput).
     const int64_t pstride = (int64_t)2 * a.nchan * 64 * 4;
@@ -278,29 +264,31 @@ __global__ void __launch_bounds__(corr::kThreads, 1) corr_kernel(CorrArgs a) {
 // Channel-major correlator.  Input [nchan][npkt][64 ant][4 B] (one contiguous
 // stream per channel, written by reorder_cm_kernel).
 //
-// Per 64-packet stage and time slot t, two K-major SWIZZLE_64B operand
-// tiles of 128 rows (2 ant + pol) x 64 bytes, R then I (8 KB each, so that
-// [R; I] is one 256-row operand), with packet P at K byte 8 (P mod 8) + P / 8
-// (a permutation shared by every operand).  Two MMA groups per slot:
+// Per 64-packet stage and time slot t, two MN-major SWIZZLE_128B operand
+// tiles, R then I, of 64 packets (K) x 128 bytes (row s = 2 ant + pol), 8 KB
+// each, so that [R; I] is one 256-row operand.  Two MMA groups per slot:
 //     R [R; I]^T   (N = 256, K = 64)  -> R R^T | R I^T   TMEM cols t*256 + [0, 256)
 //     I I^T        (N = 128, K = 64)  += into cols t*256 + [0, 128)
 // so cols [0, 128) hold Re = R R^T + I I^T and cols [128, 256) hold
 // E = R I^T = C^T for C = I R^T; the epilogue forms Im = C - C^T from E and
-// its transpose (through shared memory).  The tensor time equals one N = 128
-// group per 32 bytes of K; the operand reads are 80 KB per stage (a single
-// [R | I] tile with Re = A A^T and C = I R^T as four and two N = 128 MMAs
-// read 96 KB).
-// Thread (antenna, c) owns the 16 packets P = 2c + e + 8q (e = 0, 1;
-// q = 0..7), i.e. 16-byte chunk c of the R and of the I tile.  Its 16 words come either
-// straight from global memory (kBulk = false: lanes = consecutive
-// antennas, coalesced, two stages ahead in registers) or from 16 KB stages
-// that a loader warp brings in with one cp.async.bulk each, four ahead
-// (kBulk = true; conflict-free shared reads).  It transposes bytes with
-// prmt and sign-extends nibbles with carry-free bytewise adds.  Lanes 4..7 of each group of 8
-// store the two pols in the opposite order, so every 16-byte store
-// instruction covers all eight bank groups (the 64-byte swizzle spreads
-// four consecutive antennas' chunks over four groups, the pol the other
-// four).
+// its transpose (through shared memory).  The operand reads are 80 KB per
+// stage (a single [R | I] tile with Re = A A^T and C = I R^T as four and two
+// N = 128 MMAs read 96 KB).
+// A packet's samples are already consecutive in M, so with MN-major operands
+// the unpack is bytewise: one prmt per four bytes separates the time slots,
+// and the operands are 16 times the nibbles (two and one operations per four
+// samples), the products 256 times the visibilities, divided out exactly in
+// the epilogue.  (K-major tiles needed 4x4 byte transposes and sign
+// extension, and one mbarrier arrival per thread instead of per warp: 97
+// against 76 us for the full block; what is left is 46 us of MMAs alone and
+// the epilogue.)
+// Thread (packet P, octet o of 8 antennas = 32 bytes = chunk o of the tile
+// rows) loads two 16-byte halves and stores one 16-byte chunk to each of the
+// four tiles.  Octets 4..7 load (and keep) their halves swapped, so that the
+// eight lanes of a packet cover all banks; ant_of undoes that permutation of
+// the operand rows in the epilogue.  The halves come either straight from
+// global memory (FEED 0: two stages ahead in registers) or from 16 KB stages
+// that a loader warp brings in, four ahead.
 // Persistent (FEED 0 / 1): one CTA per SM, each correlating channels
 // blockIdx.x, + gridDim.x, ...; the raw and operand rings and their
 // barrier phases run on across a CTA's channels, so the loader brings the
@@ -313,14 +301,15 @@ __global__ void __launch_bounds__(corr::kThreads, 1) corr_kernel(CorrArgs a) {
 // written by TMEM lane quadrant I, except block (3, 0), which quadrant 0
 // writes as the conjugates of its own rows, so that no warp writes more
 // than three blocks (four before).
-// NW = 16 (bulk-fed only) doubles the unpack warps: warps 8..15 repeat the
-// mapping of warps 0..7 for time slot 1 while warps 0..7 take slot 0 (each
-// raw word is read twice, each thread does half the byte work), and the
-// epilogue splits every warp's column blocks between the two halves.
+// NW = 16 (bulk-fed only) doubles the unpack warps (one packet per thread
+// and stage instead of two), and the epilogue splits every warp's column
+// blocks between the two halves.
 //
 // Feeds (FEED): 0 direct loads and 1 one bulk copy per stage, both from the
-// channel-major corner turn; 2 the captured block itself, with no corner
-// turn.  FEED 2 runs in clusters of four CTAs, the four channels of one
+// channel-major corner turn; 3 one TMA box per stage from the REORDER-key
+// block (its rows are already separate per time slot: no prmt, no
+// permutation); 2 the captured block itself, with no corner turn.  FEED 2
+// runs in clusters of four CTAs, the four channels of one
 // 16-byte row of the captured layout.  Per 64-packet stage, CTA r of the
 // cluster loads one TMA box [16 packets][nant_in antennas][16 bytes]
 // (packets 16r..16r+15 of the stage, all four channels; rows past the
@@ -355,26 +344,37 @@ template <int FEED> constexpr int raw_stages() { return FEED == 2 ? 3 : 4; }
 // NW unpack/epilogue warps + UMMA warp (+ bulk loader warp for FEED 1; TMA
 // warp, raw-slot manager warp and two transposer warps for FEED 2)
 template <int FEED, int NW> constexpr int threads() {
-  return 32 * NW + 32 + (FEED == 1 ? 32 : FEED == 2 ? 128 : 0);
+  return 32 * NW + 32 + (FEED == 1 || FEED == 3 ? 32 : FEED == 2 ? 128 : 0);
 }
 template <int FEED> constexpr int smem_bytes() {
   return 1024 + kOpStages * kStageBytes + (FEED >= 1 ? raw_stages<FEED>() * kRawBytes : 0) +
          (FEED == 2 ? raw_stages<FEED>() * kLandBytes : 0);
 }
-constexpr uint32_t kIdescN128 = umma_idesc(/*S32*/ 2, /*s8*/ 1, /*s8*/ 1, 128, 128);
-constexpr uint32_t kIdescN256 = umma_idesc(/*S32*/ 2, /*s8*/ 1, /*s8*/ 1, 128, 256);
-constexpr uint32_t kHalfTile = 128 * 64;           // one 64-byte-row tile (R or I)
+constexpr uint32_t kIdescN128 = umma_idesc(/*S32*/ 2, /*s8*/ 1, /*s8*/ 1, 128, 128) | kIdescMnMajor;
+constexpr uint32_t kIdescN256 = umma_idesc(/*S32*/ 2, /*s8*/ 1, /*s8*/ 1, 128, 256) | kIdescMnMajor;
+constexpr uint32_t kHalfTile = kPktPerStage * 128; // one tile (R or I) of a time slot
 static_assert(kOpStages * kStageBytes >= 2 * 128 * 128 * 4, "C^T scratch reuses the stages");
 }  // namespace corrcm
 
-// Low / high nibble of each byte (4-bit two's complement) -> int8, bytewise
-// without carries: x = nibble ^ 8 = v + 8 in [0, 15]; (x + 0x78) ^ 0x80 = v.
-__device__ __forceinline__ uint32_t sext_lo4(uint32_t w) {
-  return (((w & 0x0F0F0F0Fu) ^ 0x08080808u) + 0x78787878u) ^ 0x80808080u;
+// 16 times the low / high nibble (4-bit two's complement) of each byte, as
+// int8: the nibble in the byte's upper half is its own sign extension.
+__device__ __forceinline__ uint32_t x16_lo(uint32_t w) { return (w << 4) & 0xF0F0F0F0u; }
+__device__ __forceinline__ uint32_t x16_hi(uint32_t w) { return w & 0xF0F0F0F0u; }
+
+// The sums of products of the 16-fold operands are 256 times the
+// visibilities: at most 2^31 for 65,536 packets, reached only by the real
+// part of an autocorrelation of -8 - 8i throughout, which wraps to the
+// lowest int32 (no other sum can reach it); everything else is exact in
+// FP32 (multiples of 256 below 2^31).
+__device__ __forceinline__ float vis_re(uint32_t v) {
+  return v == 0x80000000u ? 8388608.0f : (float)(int32_t)v * 0.00390625f;
 }
-__device__ __forceinline__ uint32_t sext_hi4(uint32_t w) {
-  return ((((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u) + 0x78787878u) ^ 0x80808080u;
-}
+__device__ __forceinline__ float vis_im(int32_t v) { return (float)v * 0.00390625f; }
+
+// Antenna of operand slot s (row pairs of a tile): with kPerm the halves of
+// the upper four octets are swapped.
+template <bool kPerm>
+__device__ __forceinline__ int ant_of(int s) { return kPerm && s >= 32 ? s ^ 4 : s; }
 
 template <int FEED, int NW>
 __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
@@ -382,6 +382,8 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
   using namespace corrcm;
   constexpr bool kBulk = FEED >= 1;   // unpack from raw stages in shared memory
   constexpr bool kCl = FEED == 2;
+  constexpr bool kPerm = FEED != 3;   // upper octets stored with their halves swapped
+  constexpr int kUnits = 16 / NW;     // packets per unpack thread and stage
   constexpr int kRawStages = raw_stages<FEED>();
   static_assert(NW == 8 || (NW == 16 && kBulk), "8 unpack warps, or 16 when stage-fed");
   constexpr int kUnpackThreads = 32 * NW;
@@ -410,12 +412,12 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
 
   if (tid == 0) {
     for (int s = 0; s < kOpStages; ++s) {
-      mbar_init(&full_bar[s], kUnpackThreads);
+      mbar_init(&full_bar[s], NW);
       mbar_init(&empty_bar[s], 1);
     }
     for (int r = 0; r < kRawStages; ++r) {
       mbar_init(&rfull_bar[r], 1);
-      mbar_init(&rempty_bar[r], kUnpackThreads);
+      mbar_init(&rempty_bar[r], NW);
     }
     mbar_init(&accum_bar, 1);
     mbar_init(&final_bar, 1);
@@ -448,121 +450,98 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
 
   if (warp < NW) {
     // ------------------------------------------------------------ unpack
-    const int ant = lane + 32 * (warp & 1);
-    const uint32_t c = (uint32_t)((warp >> 1) & 3);    // 16-byte chunk of each half (0..3)
-    const int tsel = warp >> 3;                        // NW = 16: the one time slot
-    const uint32_t flip = (uint32_t)(lane >> 2) & 1u;  // store pol 1 first
-    // tile offsets of this thread's chunks, store order sp = 0, 1 (pol = sp ^ flip)
-    uint32_t o_re[2], o_im[2];
-#pragma unroll
-    for (int sp = 0; sp < 2; ++sp) {
-      const uint32_t row = (uint32_t)(2 * ant) + ((uint32_t)sp ^ flip);
-      o_re[sp] = sw64_offset(row, c);
-      o_im[sp] = kHalfTile + sw64_offset(row, c);
-    }
+    const uint32_t o = (uint32_t)lane & 7u;            // 16-byte operand chunk of the thread
+    const int p_thr = 4 * kUnits * warp + (lane >> 3); // its first packet of a stage
+    const uint32_t h0 = kPerm ? (o >> 2) & 1u : 0u;    // 16-byte half loaded first
     int gs0 = 0;                                       // stages of the earlier channels
-    const uint32_t *chan_src = nullptr;                // FEED 0: the channel's stream
-    // w[e][q]: packet 2c + e + 8q of the stage, word = bytes [t0p0, t0p1, t1p0, t1p1]
-    auto load = [&](int ks, uint32_t (&w)[2][8]) {
+    const uint4 *chan_src = nullptr;                   // FEED 0: the channel's stream
+    // the two 16-byte words of packet row `row` (256 bytes = 16 words): FEED 3
+    // chunk o of each time slot, else the chunk's eight antennas
+    const uint32_t i0 = FEED == 3 ? o : 2u * o + h0;
+    const uint32_t i1 = FEED == 3 ? o + 8u : 2u * o + (h0 ^ 1u);
+    auto load = [&](int ks, uint4 (&w)[kUnits][2]) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int p = ks * kPktPerStage + 2 * (int)c + e + 8 * q;
-          w[e][q] = (ks < nks && p < a.npkt) ? __ldg(chan_src + (int64_t)p * 64 + ant) : 0u;
-        }
+      for (int u = 0; u < kUnits; ++u) {
+        const int p = ks * kPktPerStage + p_thr + 4 * u;
+        const bool ok = ks < nks && p < a.npkt;
+        w[u][0] = ok ? __ldg(chan_src + (int64_t)p * 16 + i0) : make_uint4(0u, 0u, 0u, 0u);
+        w[u][1] = ok ? __ldg(chan_src + (int64_t)p * 16 + i1) : make_uint4(0u, 0u, 0u, 0u);
+      }
     };
-    auto unpack_store = [&](int ks, const uint32_t (&w)[2][8]) -> bool {
+    auto unpack_store = [&](int ks, const uint4 (&w)[kUnits][2]) -> bool {
       const int G = gs0 + ks;
       const int s = G % kOpStages;
-      if (!mbar_wait_bounded(&empty_bar[s], ((uint32_t)(G / kOpStages) & 1u) ^ 1u, &abort_sh,
-                             a.err, DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
-        return false;
-      // X[sl][e][h]: sample slot sl = 2t + pol of packets q = 4h .. 4h+3
-      // (NW = 16: only the slots of time slot tsel, at sl = 0, 1)
-      uint32_t X[4][2][2];
-      const uint32_t sel_t = tsel ? 0x7362u : 0x5140u;
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint32_t *v = &w[e][4 * h];
-          if (NW == 16) {
-            const uint32_t ta = __byte_perm(v[0], v[1], sel_t);
-            const uint32_t tb = __byte_perm(v[2], v[3], sel_t);
-            X[0][e][h] = __byte_perm(ta, tb, 0x5410u);
-            X[1][e][h] = __byte_perm(ta, tb, 0x7632u);
-          } else {
-            const uint32_t t0 = __byte_perm(v[0], v[1], 0x5140u);
-            const uint32_t t1 = __byte_perm(v[0], v[1], 0x7362u);
-            const uint32_t t2 = __byte_perm(v[2], v[3], 0x5140u);
-            const uint32_t t3 = __byte_perm(v[2], v[3], 0x7362u);
-            X[0][e][h] = __byte_perm(t0, t2, 0x5410u);
-            X[1][e][h] = __byte_perm(t0, t2, 0x7632u);
-            X[2][e][h] = __byte_perm(t1, t3, 0x5410u);
-            X[3][e][h] = __byte_perm(t1, t3, 0x7632u);
-          }
-        }
+      const bool ok = mbar_wait_bounded(&empty_bar[s], ((uint32_t)(G / kOpStages) & 1u) ^ 1u,
+                                        &abort_sh, a.err, DEV_ERR_WAIT_EMPTY, a.wait_limit_ns);
+      if (!__all_sync(0xffffffffu, ok)) return false;
       const uint32_t stage = sbase + (uint32_t)s * kStageBytes;
 #pragma unroll
-      for (int tt = 0; tt < (NW == 16 ? 1 : 2); ++tt) {
-        const int t = NW == 16 ? tsel : tt;   // time slot (tile)
-        const int xs = 2 * tt;                // its slots in X
+      for (int u = 0; u < kUnits; ++u) {
+        const uint32_t P = (uint32_t)(p_thr + 4 * u);
+        const uint32_t dst = stage + P * 128u + ((o ^ (P & 7u)) << 4);
+        uint32_t x[2][4];   // the chunk of each time slot, packed
+        if (FEED == 3) {
+          x[0][0] = w[u][0].x; x[0][1] = w[u][0].y; x[0][2] = w[u][0].z; x[0][3] = w[u][0].w;
+          x[1][0] = w[u][1].x; x[1][1] = w[u][1].y; x[1][2] = w[u][1].z; x[1][3] = w[u][1].w;
+        } else {            // antenna words [t0p0, t0p1, t1p0, t1p1]
 #pragma unroll
-        for (int sp = 0; sp < 2; ++sp) {
-          const uint32_t pol = (uint32_t)sp ^ flip;
-          uint32_t re[4], im[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {   // chunk word k = (e, h) = (k >> 1, k & 1)
-            const uint32_t x0 = X[xs][k >> 1][k & 1], x1 = X[xs + 1][k >> 1][k & 1];
-            const uint32_t x = pol ? x1 : x0;
-            re[k] = sext_lo4(x);
-            im[k] = sext_hi4(x);
+          for (int t = 0; t < 2; ++t) {
+            const uint32_t sel = t ? 0x7632u : 0x5410u;
+            x[t][0] = __byte_perm(w[u][0].x, w[u][0].y, sel);
+            x[t][1] = __byte_perm(w[u][0].z, w[u][0].w, sel);
+            x[t][2] = __byte_perm(w[u][1].x, w[u][1].y, sel);
+            x[t][3] = __byte_perm(w[u][1].z, w[u][1].w, sel);
           }
-          const uint32_t tile = stage + (uint32_t)t * kTile;
-          st_shared_v4(tile + o_re[sp], re[0], re[1], re[2], re[3]);
-          st_shared_v4(tile + o_im[sp], im[0], im[1], im[2], im[3]);
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t d = dst + (uint32_t)t * kTile;
+          st_shared_v4(d, x16_lo(x[t][0]), x16_lo(x[t][1]), x16_lo(x[t][2]), x16_lo(x[t][3]));
+          st_shared_v4(d + kHalfTile, x16_hi(x[t][0]), x16_hi(x[t][1]), x16_hi(x[t][2]),
+                       x16_hi(x[t][3]));
         }
       }
       fence_proxy_async_smem();
-      mbar_arrive(&full_bar[s]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[s]);
       return true;
     };
-    const uint32_t *rw_base = reinterpret_cast<const uint32_t *>(gbase + kOpStages * kStageBytes);
+    const uint4 *rw_base = reinterpret_cast<const uint4 *>(gbase + kOpStages * kStageBytes);
     // the words of raw stage ks -> w, then the stage goes back to the loader
-    auto fetch = [&](int ks, uint32_t (&w)[2][8]) -> bool {
+    auto fetch = [&](int ks, uint4 (&w)[kUnits][2]) -> bool {
       const int G = gs0 + ks;
       const int r = G % kRawStages;
-      if (!mbar_wait_bounded<kCl>(&rfull_bar[r], (uint32_t)(G / kRawStages) & 1u, &abort_sh,
-                                  a.err, DEV_ERR_WAIT_FULL, a.wait_limit_ns))
-        return false;
-      const uint32_t *rw = rw_base + r * (kRawBytes / 4);
+      const bool ok = mbar_wait_bounded<kCl>(&rfull_bar[r], (uint32_t)(G / kRawStages) & 1u, &abort_sh,
+                                             a.err, DEV_ERR_WAIT_FULL, a.wait_limit_ns);
+      if (!__all_sync(0xffffffffu, ok)) return false;
+      const uint4 *rw = rw_base + r * (kRawBytes / 16);
       const int pvalid = a.npkt - ks * kPktPerStage;
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int P = 2 * (int)c + e + 8 * q;
-          w[e][q] = P < pvalid ? rw[P * 64 + ant] : 0u;
-        }
+      for (int u = 0; u < kUnits; ++u) {
+        const int P = p_thr + 4 * u;
+        const bool live = FEED == 3 || P < pvalid;   // (FEED 3's boxes are zero past the block)
+        w[u][0] = live ? rw[P * 16 + i0] : make_uint4(0u, 0u, 0u, 0u);
+        w[u][1] = live ? rw[P * 16 + i1] : make_uint4(0u, 0u, 0u, 0u);
+      }
       // The next bulk copy (async proxy) overwrites this stage: order these
       // generic-proxy reads before it, or under load the copy can land
       // first (a write-after-read race across proxies).
       fence_proxy_async_smem();
-      mbar_arrive(&rempty_bar[r]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&rempty_bar[r]);
       return true;
     };
 #pragma unroll 1
     for (int ci = 0; ci < nchc; ++ci) {
       const int ch = (int)blockIdx.x + ci * (kCl ? 0 : (int)gridDim.x);
       gs0 = ci * nks;
-      chan_src = reinterpret_cast<const uint32_t *>(a.in + (int64_t)ch * a.npkt * 256);
+      chan_src = reinterpret_cast<const uint4 *>(a.in + (int64_t)ch * a.npkt * 256);
       if (kBulk) {
         // one stage of words in registers ahead of the stage being unpacked,
         // so the shared-memory loads overlap the previous stage's unpack
-        uint32_t wa[2][8], wb[2][8];
+        uint4 wa[kUnits][2], wb[kUnits][2];
         if (nks > 0 && fetch(0, wa)) {
-          for (int ks = 0; ks < nks && !abort_sh; ks += 2) {
+          for (int ks = 0; ks < nks; ks += 2) {
             if (ks + 1 < nks && !fetch(ks + 1, wb)) break;
             if (!unpack_store(ks, wa)) break;
             if (ks + 1 >= nks) break;
@@ -572,10 +551,10 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
         }
       } else {
         // two stages of loads in flight ahead of the stage being unpacked
-        uint32_t wa[2][8], wb[2][8], wc[2][8];
+        uint4 wa[kUnits][2], wb[kUnits][2], wc[kUnits][2];
         load(0, wa);
         load(1, wb);
-        for (int ks = 0; ks < nks && !abort_sh; ks += 3) {
+        for (int ks = 0; ks < nks; ks += 3) {
           load(ks + 2, wc);
           if (!unpack_store(ks, wa)) break;
           if (ks + 1 >= nks) break;
@@ -612,7 +591,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
       }
       named_bar(1, kUnpackThreads);
       if (ok) {
-        const int i = m >> 1, pi = m & 1;
+        const int i = ant_of<kPerm>(m >> 1), pi = m & 1;
         float *vis = a.vis + (int64_t)(2 * ch + t) * (2080 * 8);
         const int64_t tri = (int64_t)i * (i + 1) / 2;
         const int ncb = 2 * q + 2;
@@ -628,15 +607,14 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
           tmem_wait_ld();
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
-            const int j = 8 * cb + jj;
+            const int j = ant_of<kPerm>(8 * cb + jj);
             if (j <= i) {
-              const int b0 = 2 * j, b1 = 2 * j + 1;
+              const int b0 = 2 * (8 * cb + jj), b1 = b0 + 1;
               const int32_t ct0 = (int32_t)Cs[b0 * 128 + (m ^ (b0 & 31))];
               const int32_t ct1 = (int32_t)Cs[b1 * 128 + (m ^ (b1 & 31))];
               // cr = E[m][.] = C[.][m], ct = C[m][.]: Im = C[m][.] - C[.][m]
-              float4 o = make_float4((float)(int32_t)re[2 * jj], (float)(ct0 - (int32_t)cr[2 * jj]),
-                                     (float)(int32_t)re[2 * jj + 1],
-                                     (float)(ct1 - (int32_t)cr[2 * jj + 1]));
+              float4 o = make_float4(vis_re(re[2 * jj]), vis_im(ct0 - (int32_t)cr[2 * jj]),
+                                     vis_re(re[2 * jj + 1]), vis_im(ct1 - (int32_t)cr[2 * jj + 1]));
               float4 *dst = reinterpret_cast<float4 *>(vis + ((tri + j) * 4 + 2 * pi) * 2);
               if (a.accumulate) {
                 const float4 old = *dst;
@@ -659,13 +637,12 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
             tmem_wait_ld();
 #pragma unroll
             for (int ii = 0; ii < 8; ++ii) {
-              const int ic = 48 + 8 * ib + ii;   // output row antenna i
-              const int n0 = 2 * ic, n1 = 2 * ic + 1;
+              const int ic = ant_of<kPerm>(48 + 8 * ib + ii);   // output row antenna i
+              const int n0 = 2 * (48 + 8 * ib + ii), n1 = n0 + 1;
               const int32_t en0 = (int32_t)Cs[n0 * 128 + (m ^ (n0 & 31))];   // E[n0][m']
               const int32_t en1 = (int32_t)Cs[n1 * 128 + (m ^ (n1 & 31))];
-              const float r0 = (float)(int32_t)re[2 * ii], i0 = (float)((int32_t)er[2 * ii] - en0);
-              const float r1 = (float)(int32_t)re[2 * ii + 1],
-                          i1 = (float)((int32_t)er[2 * ii + 1] - en1);
+              const float r0 = vis_re(re[2 * ii]), i0 = vis_im((int32_t)er[2 * ii] - en0);
+              const float r1 = vis_re(re[2 * ii + 1]), i1 = vis_im((int32_t)er[2 * ii + 1] - en1);
               // pj = 0 keeps pi = 0 and sends pi = 1; pj = 1 the reverse
               const float sr = __shfl_xor_sync(0xffffffffu, pj ? r0 : r1, 1);
               const float si = __shfl_xor_sync(0xffffffffu, pj ? i0 : i1, 1);
@@ -799,7 +776,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
                            cluster_map(&rfull_bar[r], q));
       }
     }
-  } else if (FEED == 1 && warp == NW + 1) {
+  } else if ((FEED == 1 || FEED == 3) && warp == NW + 1) {
     // ------------------------------------------------------------ bulk loader
     if (lane == 0) {
       // the stages of all the CTA's channels in order: the next channel's
@@ -812,6 +789,12 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
         if (!mbar_wait_bounded(&rempty_bar[r], ((uint32_t)(G / kRawStages) & 1u) ^ 1u, &abort_sh,
                                a.err, DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
           break;
+        if (FEED == 3) {   // the stage's packets x 256 bytes (both time slots) as one box
+          mbar_arrive_expect_tx(&rfull_bar[r], kRawBytes);
+          tma_load_2d(raw_base + (uint32_t)r * kRawBytes, &tmap, 256 * chg, ks * kPktPerStage,
+                      &rfull_bar[r]);
+          continue;
+        }
         const int npk = min(kPktPerStage, a.npkt - ks * kPktPerStage);
         const uint32_t bytes = (uint32_t)npk * 256u;
         mbar_arrive_expect_tx(&rfull_bar[r], bytes);
@@ -852,13 +835,13 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
           const uint32_t tr = stage + (uint32_t)t * kTile, ti = tr + kHalfTile;
           const uint32_t dre = tmem + (uint32_t)t * 256u;
 #pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {   // R [R; I]^T: K = 64 bytes = 2 x 32
-            const uint64_t d = umma_desc_sw64(tr + 32u * kk, 512u);
+          for (int kk = 0; kk < 2; ++kk) {   // R [R; I]^T: K = 64 packets = 2 x 32
+            const uint64_t d = umma_desc_mn128(tr + 4096u * kk, kHalfTile, 1024u);
             umma_i8(dre, d, d, kIdescN256, (ks | kk) != 0);
           }
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk) {   // += I I^T into the first 128 columns
-            const uint64_t d = umma_desc_sw64(ti + 32u * kk, 512u);
+            const uint64_t d = umma_desc_mn128(ti + 4096u * kk, kHalfTile, 1024u);
             umma_i8(dre, d, d, kIdescN128, 1u);
           }
         }
@@ -903,6 +886,22 @@ static int encode_captured_map(CUtensorMap *map, const CorrArgs &a) {
   return r == CUDA_SUCCESS ? 0 : -1;
 }
 
+// FEED 3: the REORDER-key block [npkt][nchan][256 B] as a 2-D uint8 tensor
+// of packet rows; boxes of 64 packets x one channel's 256 bytes.
+static int encode_reordered_map(CUtensorMap *map, const CorrArgs &a) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (!fn) return -1;
+  const cuuint64_t dims[2] = {(cuuint64_t)a.nchan * 256, (cuuint64_t)a.npkt};
+  const cuuint64_t strides[1] = {(cuuint64_t)a.nchan * 256};
+  const cuuint32_t box[2] = {256u, (cuuint32_t)corrcm::kPktPerStage};
+  const cuuint32_t estr[2] = {1u, 1u};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(a.in), dims,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -1;
+}
+
 template <int FEED, int NW>
 static int launch_cm(const CorrArgs &a, cudaStream_t st) {
   static SmemAttrOnce attr;
@@ -911,6 +910,7 @@ static int launch_cm(const CorrArgs &a, cudaStream_t st) {
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   if (FEED == 2 && encode_captured_map(&tmap, a) != 0) return -2;
+  if (FEED == 3 && encode_reordered_map(&tmap, a) != 0) return -2;
   cudaLaunchConfig_t cfg = {};
   // FEED 0 / 1: persistent, one CTA per SM (the 512 TMEM columns), each
   // looping over channels blockIdx.x, + gridDim.x, ...; FEED 2: one CTA
@@ -965,10 +965,10 @@ int launch_correlate_captured_cluster(const CorrArgs &a, cudaStream_t st, int un
 
 int launch_correlate(const CorrArgs &a, int fmt, cudaStream_t st) {
   static SmemAttrOnce attr[3];
-  const void *fn = fmt == FMT_CAPTURED    ? (const void *)corr_kernel<FMT_CAPTURED>
-                   : fmt == FMT_REORDERED ? (const void *)corr_kernel<FMT_REORDERED>
-                                          : (const void *)corr_kernel<FMT_XGPU_INT8>;
   if (fmt < 0 || fmt > 2) return -1;
+  if (fmt == FMT_REORDERED) return launch_cm<3, 8>(a, st);
+  const void *fn = fmt == FMT_CAPTURED ? (const void *)corr_kernel<FMT_CAPTURED>
+                                       : (const void *)corr_kernel<FMT_XGPU_INT8>;
   if (smem_attr_once(attr[fmt], fn, corr::kSmemBytes) != cudaSuccess) return -2;
   dim3 grid(a.nchan), block(corr::kThreads);
   void *args[] = {(void *)&a};
