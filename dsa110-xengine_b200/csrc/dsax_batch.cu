@@ -45,12 +45,12 @@ int enqueue_block(dsax_ctx *c, const dsax_block_desc &d, uint8_t *scratch, float
       if (launch_correlate_captured_cluster(a, sc, corr_path_unpack_warps(cf.corr_path)) != 0)
         return -2;
     } else {
-      if (launch_reorder_chanmajor(static_cast<const uint8_t *>(d.blk), scratch, npkt, cf.nant_in,
-                                   nchan, sc) != 0)
+      if (launch_corner_turn(static_cast<const uint8_t *>(d.blk), scratch, npkt, cf.nant_in, nchan, sc,
+                             cf.corr_path) != 0)
         return -2;
       a.in = scratch;
       a.nant_in = 64;
-      if (launch_correlate_chanmajor(a, sc, cf.corr_path) != 0) return -2;
+      if (launch_correlate_turned(a, sc, cf.corr_path) != 0) return -2;
     }
   }
   if (d.beams || d.chanmask) {

@@ -306,10 +306,8 @@ __global__ void __launch_bounds__(corr::kThreads, 1) corr_kernel(CorrArgs a) {
 // blocks between the two halves.
 //
 // Feeds (FEED): 0 direct loads and 1 one bulk copy per stage, both from the
-// channel-major corner turn; 3 one TMA box per stage from the REORDER-key
-// block (its rows are already separate per time slot: no prmt, no
-// permutation); 2 the captured block itself, with no corner turn.  FEED 2
-// runs in clusters of four CTAs, the four channels of one
+// channel-major corner turn; 2 the captured block itself, with no corner
+// turn.  FEED 2 runs in clusters of four CTAs, the four channels of one
 // 16-byte row of the captured layout.  Per 64-packet stage, CTA r of the
 // cluster loads one TMA box [16 packets][nant_in antennas][16 bytes]
 // (packets 16r..16r+15 of the stage, all four channels; rows past the
@@ -344,7 +342,7 @@ template <int FEED> constexpr int raw_stages() { return FEED == 2 ? 3 : 4; }
 // NW unpack/epilogue warps + UMMA warp (+ bulk loader warp for FEED 1; TMA
 // warp, raw-slot manager warp and two transposer warps for FEED 2)
 template <int FEED, int NW> constexpr int threads() {
-  return 32 * NW + 32 + (FEED == 1 || FEED == 3 ? 32 : FEED == 2 ? 128 : 0);
+  return 32 * NW + 32 + (FEED == 1 ? 32 : FEED == 2 ? 128 : 0);
 }
 template <int FEED> constexpr int smem_bytes() {
   return 1024 + kOpStages * kStageBytes + (FEED >= 1 ? raw_stages<FEED>() * kRawBytes : 0) +
@@ -356,25 +354,9 @@ constexpr uint32_t kHalfTile = kPktPerStage * 128; // one tile (R or I) of a tim
 static_assert(kOpStages * kStageBytes >= 2 * 128 * 128 * 4, "C^T scratch reuses the stages");
 }  // namespace corrcm
 
-// 16 times the low / high nibble (4-bit two's complement) of each byte, as
-// int8: the nibble in the byte's upper half is its own sign extension.
-__device__ __forceinline__ uint32_t x16_lo(uint32_t w) { return (w << 4) & 0xF0F0F0F0u; }
-__device__ __forceinline__ uint32_t x16_hi(uint32_t w) { return w & 0xF0F0F0F0u; }
-
-// The sums of products of the 16-fold operands are 256 times the
-// visibilities: at most 2^31 for 65,536 packets, reached only by the real
-// part of an autocorrelation of -8 - 8i throughout, which wraps to the
-// lowest int32 (no other sum can reach it); everything else is exact in
-// FP32 (multiples of 256 below 2^31).
-__device__ __forceinline__ float vis_re(uint32_t v) {
-  return v == 0x80000000u ? 8388608.0f : (float)(int32_t)v * 0.00390625f;
-}
-__device__ __forceinline__ float vis_im(int32_t v) { return (float)v * 0.00390625f; }
-
-// Antenna of operand slot s (row pairs of a tile): with kPerm the halves of
-// the upper four octets are swapped.
-template <bool kPerm>
-__device__ __forceinline__ int ant_of(int s) { return kPerm && s >= 32 ? s ^ 4 : s; }
+// Antenna of operand slot s (row pairs of a tile): the halves of the upper
+// four octets are swapped.
+__device__ __forceinline__ int ant_of(int s) { return s >= 32 ? s ^ 4 : s; }
 
 template <int FEED, int NW>
 __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
@@ -382,7 +364,6 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
   using namespace corrcm;
   constexpr bool kBulk = FEED >= 1;   // unpack from raw stages in shared memory
   constexpr bool kCl = FEED == 2;
-  constexpr bool kPerm = FEED != 3;   // upper octets stored with their halves swapped
   constexpr int kUnits = 16 / NW;     // packets per unpack thread and stage
   constexpr int kRawStages = raw_stages<FEED>();
   static_assert(NW == 8 || (NW == 16 && kBulk), "8 unpack warps, or 16 when stage-fed");
@@ -452,13 +433,11 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
     // ------------------------------------------------------------ unpack
     const uint32_t o = (uint32_t)lane & 7u;            // 16-byte operand chunk of the thread
     const int p_thr = 4 * kUnits * warp + (lane >> 3); // its first packet of a stage
-    const uint32_t h0 = kPerm ? (o >> 2) & 1u : 0u;    // 16-byte half loaded first
+    const uint32_t h0 = (o >> 2) & 1u;    // 16-byte half loaded first
     int gs0 = 0;                                       // stages of the earlier channels
     const uint4 *chan_src = nullptr;                   // FEED 0: the channel's stream
-    // the two 16-byte words of packet row `row` (256 bytes = 16 words): FEED 3
-    // chunk o of each time slot, else the chunk's eight antennas
-    const uint32_t i0 = FEED == 3 ? o : 2u * o + h0;
-    const uint32_t i1 = FEED == 3 ? o + 8u : 2u * o + (h0 ^ 1u);
+    // the octet's two 16-byte words of a packet row (256 bytes = 16 words)
+    const uint32_t i0 = 2u * o + h0, i1 = 2u * o + (h0 ^ 1u);
     auto load = [&](int ks, uint4 (&w)[kUnits][2]) {
 #pragma unroll
       for (int u = 0; u < kUnits; ++u) {
@@ -480,18 +459,13 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
         const uint32_t P = (uint32_t)(p_thr + 4 * u);
         const uint32_t dst = stage + P * 128u + ((o ^ (P & 7u)) << 4);
         uint32_t x[2][4];   // the chunk of each time slot, packed
-        if (FEED == 3) {
-          x[0][0] = w[u][0].x; x[0][1] = w[u][0].y; x[0][2] = w[u][0].z; x[0][3] = w[u][0].w;
-          x[1][0] = w[u][1].x; x[1][1] = w[u][1].y; x[1][2] = w[u][1].z; x[1][3] = w[u][1].w;
-        } else {            // antenna words [t0p0, t0p1, t1p0, t1p1]
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const uint32_t sel = t ? 0x7632u : 0x5410u;
-            x[t][0] = __byte_perm(w[u][0].x, w[u][0].y, sel);
-            x[t][1] = __byte_perm(w[u][0].z, w[u][0].w, sel);
-            x[t][2] = __byte_perm(w[u][1].x, w[u][1].y, sel);
-            x[t][3] = __byte_perm(w[u][1].z, w[u][1].w, sel);
-          }
+        for (int t = 0; t < 2; ++t) {   // antenna words [t0p0, t0p1, t1p0, t1p1]
+          const uint32_t sel = t ? 0x7632u : 0x5410u;
+          x[t][0] = __byte_perm(w[u][0].x, w[u][0].y, sel);
+          x[t][1] = __byte_perm(w[u][0].z, w[u][0].w, sel);
+          x[t][2] = __byte_perm(w[u][1].x, w[u][1].y, sel);
+          x[t][3] = __byte_perm(w[u][1].z, w[u][1].w, sel);
         }
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
@@ -519,7 +493,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
 #pragma unroll
       for (int u = 0; u < kUnits; ++u) {
         const int P = p_thr + 4 * u;
-        const bool live = FEED == 3 || P < pvalid;   // (FEED 3's boxes are zero past the block)
+        const bool live = P < pvalid;
         w[u][0] = live ? rw[P * 16 + i0] : make_uint4(0u, 0u, 0u, 0u);
         w[u][1] = live ? rw[P * 16 + i1] : make_uint4(0u, 0u, 0u, 0u);
       }
@@ -591,7 +565,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
       }
       named_bar(1, kUnpackThreads);
       if (ok) {
-        const int i = ant_of<kPerm>(m >> 1), pi = m & 1;
+        const int i = ant_of(m >> 1), pi = m & 1;
         float *vis = a.vis + (int64_t)(2 * ch + t) * (2080 * 8);
         const int64_t tri = (int64_t)i * (i + 1) / 2;
         const int ncb = 2 * q + 2;
@@ -607,7 +581,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
           tmem_wait_ld();
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
-            const int j = ant_of<kPerm>(8 * cb + jj);
+            const int j = ant_of(8 * cb + jj);
             if (j <= i) {
               const int b0 = 2 * (8 * cb + jj), b1 = b0 + 1;
               const int32_t ct0 = (int32_t)Cs[b0 * 128 + (m ^ (b0 & 31))];
@@ -637,7 +611,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
             tmem_wait_ld();
 #pragma unroll
             for (int ii = 0; ii < 8; ++ii) {
-              const int ic = ant_of<kPerm>(48 + 8 * ib + ii);   // output row antenna i
+              const int ic = ant_of(48 + 8 * ib + ii);   // output row antenna i
               const int n0 = 2 * (48 + 8 * ib + ii), n1 = n0 + 1;
               const int32_t en0 = (int32_t)Cs[n0 * 128 + (m ^ (n0 & 31))];   // E[n0][m']
               const int32_t en1 = (int32_t)Cs[n1 * 128 + (m ^ (n1 & 31))];
@@ -776,7 +750,7 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
                            cluster_map(&rfull_bar[r], q));
       }
     }
-  } else if ((FEED == 1 || FEED == 3) && warp == NW + 1) {
+  } else if (FEED == 1 && warp == NW + 1) {
     // ------------------------------------------------------------ bulk loader
     if (lane == 0) {
       // the stages of all the CTA's channels in order: the next channel's
@@ -789,12 +763,6 @@ __global__ void __launch_bounds__(corrcm::threads<FEED, NW>(), 1)
         if (!mbar_wait_bounded(&rempty_bar[r], ((uint32_t)(G / kRawStages) & 1u) ^ 1u, &abort_sh,
                                a.err, DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
           break;
-        if (FEED == 3) {   // the stage's packets x 256 bytes (both time slots) as one box
-          mbar_arrive_expect_tx(&rfull_bar[r], kRawBytes);
-          tma_load_2d(raw_base + (uint32_t)r * kRawBytes, &tmap, 256 * chg, ks * kPktPerStage,
-                      &rfull_bar[r]);
-          continue;
-        }
         const int npk = min(kPktPerStage, a.npkt - ks * kPktPerStage);
         const uint32_t bytes = (uint32_t)npk * 256u;
         mbar_arrive_expect_tx(&rfull_bar[r], bytes);
@@ -886,22 +854,6 @@ static int encode_captured_map(CUtensorMap *map, const CorrArgs &a) {
   return r == CUDA_SUCCESS ? 0 : -1;
 }
 
-// FEED 3: the REORDER-key block [npkt][nchan][256 B] as a 2-D uint8 tensor
-// of packet rows; boxes of 64 packets x one channel's 256 bytes.
-static int encode_reordered_map(CUtensorMap *map, const CorrArgs &a) {
-  EncodeTiledFn fn = tensor_map_encoder();
-  if (!fn) return -1;
-  const cuuint64_t dims[2] = {(cuuint64_t)a.nchan * 256, (cuuint64_t)a.npkt};
-  const cuuint64_t strides[1] = {(cuuint64_t)a.nchan * 256};
-  const cuuint32_t box[2] = {256u, (cuuint32_t)corrcm::kPktPerStage};
-  const cuuint32_t estr[2] = {1u, 1u};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(a.in), dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -1;
-}
-
 template <int FEED, int NW>
 static int launch_cm(const CorrArgs &a, cudaStream_t st) {
   static SmemAttrOnce attr;
@@ -910,7 +862,6 @@ static int launch_cm(const CorrArgs &a, cudaStream_t st) {
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   if (FEED == 2 && encode_captured_map(&tmap, a) != 0) return -2;
-  if (FEED == 3 && encode_reordered_map(&tmap, a) != 0) return -2;
   cudaLaunchConfig_t cfg = {};
   // FEED 0 / 1: persistent, one CTA per SM (the 512 TMEM columns), each
   // looping over channels blockIdx.x, + gridDim.x, ...; FEED 2: one CTA
@@ -953,6 +904,18 @@ int launch_correlate_chanmajor(const CorrArgs &a, cudaStream_t st, int corr_path
   }
 }
 
+int launch_corner_turn(const uint8_t *in, uint8_t *out, int npkt, int nant_in, int nchan,
+                       cudaStream_t st, int corr_path) {
+  return corr_path_chanmajor(corr_path)
+             ? launch_reorder_chanmajor(in, out, npkt, nant_in, nchan, st)
+             : launch_reorder_freqmajor(in, out, npkt, nant_in, nchan, st);
+}
+
+int launch_correlate_turned(const CorrArgs &a, cudaStream_t st, int corr_path) {
+  return corr_path_chanmajor(corr_path) ? launch_correlate_chanmajor(a, st, corr_path)
+                                        : launch_correlate_freq(a, 128, (size_t)a.npkt * 128, st);
+}
+
 bool captured_cluster_ok(const CorrArgs &a) {
   return a.nchan % corrcm::kClusterCh == 0 && a.nant_in >= 1 && a.nant_in <= 64 &&
          (reinterpret_cast<uintptr_t>(a.in) & 15u) == 0 && tensor_map_encoder() != nullptr;
@@ -966,7 +929,8 @@ int launch_correlate_captured_cluster(const CorrArgs &a, cudaStream_t st, int un
 int launch_correlate(const CorrArgs &a, int fmt, cudaStream_t st) {
   static SmemAttrOnce attr[3];
   if (fmt < 0 || fmt > 2) return -1;
-  if (fmt == FMT_REORDERED) return launch_cm<3, 8>(a, st);
+  if (fmt == FMT_REORDERED)   // [npkt][2 nchan][128 bytes]
+    return launch_correlate_freq(a, 256 * (size_t)a.nchan, 128, st);
   const void *fn = fmt == FMT_CAPTURED ? (const void *)corr_kernel<FMT_CAPTURED>
                                        : (const void *)corr_kernel<FMT_XGPU_INT8>;
   if (smem_attr_once(attr[fmt], fn, corr::kSmemBytes) != cudaSuccess) return -2;

@@ -170,6 +170,12 @@ int launch_flag_baseline(const float *hist_spec, const float *hist_var, int nave
 namespace dsax {
 int launch_reorder(const uint8_t *in, uint8_t *out, int npkt, int nant_in, int nchan,
                    cudaStream_t st);
+// The same rows as one stream per frequency: [2 nchan][npkt][64][2 pol].
+int launch_reorder_freqmajor(const uint8_t *in, uint8_t *out, int npkt, int nant_in, int nchan,
+                             cudaStream_t st);
+// Correlates frequency rows of 128 bytes [64][2 pol] at a.in + freq *
+// freq_stride + pkt * pkt_stride (both multiples of 16).
+int launch_correlate_freq(const CorrArgs &a, size_t pkt_stride, size_t freq_stride, cudaStream_t st);
 }  // namespace dsax
 
 namespace dsax {
@@ -180,6 +186,13 @@ int launch_reorder_chanmajor(const uint8_t *in, uint8_t *out, int npkt, int nant
 // registers, 5 and 7 one cp.async.bulk per 64-packet stage unpacked by 16
 // warps, anything else (4, 6) the same bulk feed unpacked by 8 warps.
 int launch_correlate_chanmajor(const CorrArgs &a, cudaStream_t st, int corr_path);
+// The corner turn of a captured block into the context's own layout (nchan *
+// npkt * 256 bytes) and the correlation from it: channel-major streams for
+// corr_path 3 and 5, frequency streams for every other one.
+inline bool corr_path_chanmajor(int corr_path) { return corr_path == 3 || corr_path == 5; }
+int launch_corner_turn(const uint8_t *in, uint8_t *out, int npkt, int nant_in, int nchan,
+                       cudaStream_t st, int corr_path);
+int launch_correlate_turned(const CorrArgs &a, cudaStream_t st, int corr_path);
 // The captured block [npkt][nant_in][nchan][4 B] correlated directly (no
 // corner turn): clusters of four channel CTAs, TMA boxes split across the
 // cluster through distributed shared memory.  Needs nchan % 4 == 0 and a

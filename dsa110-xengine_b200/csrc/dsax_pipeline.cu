@@ -5,7 +5,7 @@
 // each block's H2D copy, promote, xgpuCudaXengine and matrix copy-out
 // before it reads the next (src/dsaX_xgpu.cu:300-357).  Here block i+1's
 // corner turn (HBM-bound) runs on a side stream while block i is correlated
-// (bound by the unpack warps, with HBM bandwidth to spare), and in host mode
+// (bound by shared memory, with HBM bandwidth to spare), and in host mode
 // the PCIe copies in and out overlap both.  The fused paths (corr_path 6,
 // 7) have no corner turn: only the copies overlap the correlations.  Buffers are double-buffered and
 // every reuse waits on the event of the stage that last read the buffer.
@@ -68,13 +68,9 @@ extern "C" int dsax_correlate_many(dsax_ctx *c, const void *const *blocks, void 
   uint8_t *dvis[2] = {din[1] + up(nin), din[1] + up(nin) + up(nvis)};
 
   // The corner turns run on their own stream in both modes.  In device mode
-  // block i+1's corner turn takes the SMs that the persistent correlator's
-  // CTAs free as they finish their last channel (60 of 148 SMs idle for
-  // the last third of a 384-channel block): 0.146 against 0.162 ms per
-  // block with both on one stream.  (With one correlator CTA per channel
-  // the overlap measured slower, 0.29 against 0.165 ms: the corner turn's
-  // CTAs took the SMs the correlator's later waves needed.)  With host
-  // buffers the PCIe copies set the pace.
+  // block i+1's corner turn takes the SMs that the persistent correlator
+  // leaves (20 of 148 for 768 frequencies, and those of finished CTAs).  With
+  // host buffers the PCIe copies set the pace.
   cudaStream_t cs = c->stream, h2d = c->side[S_H2D], d2h = c->side[S_D2H];
   cudaStream_t rs = c->side[S_REO];
   cudaEvent_t *ev = c->pev;
@@ -106,7 +102,8 @@ extern "C" int dsax_correlate_many(dsax_ctx *c, const void *const *blocks, void 
       // corner turn: the correlation of block i-2 has finished reading reo[b]
       if (e == cudaSuccess && i >= 2) e = cudaStreamWaitEvent(rs, ev[E_CORR + b], 0);
       if (e != cudaSuccess) break;
-      if (launch_reorder_chanmajor(src, reo[b], c->cfg.npkt, c->cfg.nant_in, c->cfg.nchan, rs) != 0) {
+      if (launch_corner_turn(src, reo[b], c->cfg.npkt, c->cfg.nant_in, c->cfg.nchan, rs,
+                             c->cfg.corr_path) != 0) {
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaErrorInvalidValue;
         break;
@@ -126,7 +123,7 @@ extern "C" int dsax_correlate_many(dsax_ctx *c, const void *const *blocks, void 
     } else {
       a.in = reo[b];
       a.nant_in = 64;
-      lrc = launch_correlate_chanmajor(a, cs, c->cfg.corr_path);
+      lrc = launch_correlate_turned(a, cs, c->cfg.corr_path);
     }
     if (lrc != 0) {
       e = cudaGetLastError();

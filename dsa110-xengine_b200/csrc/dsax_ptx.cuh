@@ -419,4 +419,19 @@ __device__ __forceinline__ void nib8_to_bf16x8(uint32_t x, uint32_t (&o)[4]) {
   }
 }
 
+// 16 times the low / high nibble (4-bit two's complement) of each byte, as
+// int8: the nibble in the byte's upper half is its own sign extension.
+__device__ __forceinline__ uint32_t x16_lo(uint32_t w) { return (w << 4) & 0xF0F0F0F0u; }
+__device__ __forceinline__ uint32_t x16_hi(uint32_t w) { return w & 0xF0F0F0F0u; }
+
+// The sums of products of the 16-fold operands are 256 times the
+// visibilities: at most 2^31 for 65,536 packets, reached only by the real
+// part of an autocorrelation of -8 - 8i throughout, which wraps to the
+// lowest int32 (no other sum can reach it); everything else is exact in
+// FP32 (multiples of 256 below 2^31).
+__device__ __forceinline__ float vis_re(uint32_t v) {
+  return v == 0x80000000u ? 8388608.0f : (float)(int32_t)v * 0.00390625f;
+}
+__device__ __forceinline__ float vis_im(int32_t v) { return (float)v * 0.00390625f; }
+
 }  // namespace dsax

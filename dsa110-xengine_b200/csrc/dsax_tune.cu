@@ -2,10 +2,10 @@
 // a stage on the context's own geometry and device, keeps the fastest in
 // the context, and reports every timing.  Candidates for the captured-block
 // correlator (corr_path): (1) one fused kernel on the captured layout,
-// (2) corner turn to the REORDER layout + row-load correlator, (3) corner
-// turn to channel-major streams + correlator fed by direct coalesced loads,
-// (4) the same correlator fed by one bulk copy per 64-packet stage and
-// unpacked by 8 warps, (5) as 4 with 16 unpack warps, (6) no corner turn:
+// (2) corner turn to the REORDER layout + correlator over frequency rows,
+// (3) corner turn to channel-major streams + correlator fed by direct
+// coalesced loads, (4) as 2 with one stream per frequency, (5) as 3, fed by
+// one bulk copy per 64-packet stage, 16 unpack warps, (6) no corner turn:
 // the captured block read directly by clusters of four channel CTAs, (7) as
 // 6 with 16 unpack warps.  Candidates for the beamformer: (1) one CTA per
 // 64-beam tile (bf_path 1), (2-5) CTA pairs sharing a cta_group::2 MMA

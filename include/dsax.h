@@ -74,15 +74,19 @@ typedef struct dsax_config {
                             2 = corner turn to the REORDER layout + correlate,
                             3 = corner turn to channel-major streams + correlate
                                 fed by direct coalesced loads,
-                            4 = as 3, fed by one bulk copy per 64-packet stage,
-                            5 = as 4, unpacked by 16 warps instead of 8,
+                            4 = corner turn to one stream per frequency +
+                                correlate with two accumulators in turn,
+                            5 = as 3, fed by one bulk copy per 64-packet stage
+                                and unpacked by 16 warps,
                             6 = no corner turn: the correlator reads the
                                 captured block in clusters of four channel
                                 CTAs (TMA boxes split through distributed
                                 shared memory; needs nchan % 4 == 0, else 4),
                             7 = as 6, unpacked by 16 warps.
                             3 to 7 also select the feed for
-                            DSAX_FMT_CHANMAJOR (6 as 4, 7 as 5) */
+                            DSAX_FMT_CHANMAJOR: 3 direct loads, 4 and 6 bulk
+                            copies and 8 unpack warps, 5 and 7 the same with
+                            16 */
     int bf_fp8;          /* beamformer operands: 0 BF16 (tcgen05 kind::f16), 1 FP8
                             E4M3 with a per-antenna power-of-two scale
                             (kind::f8f6f4; the 4-bit data, shifted by the
@@ -162,7 +166,7 @@ int dsax_correlate(dsax_ctx *ctx, const void *in, void *vis, int mem);
  * promoter, xgpuCudaXengine, matrix copy-out, one block at a time).  Device
  * mode enqueues (ordered on the context stream); host mode returns when all
  * visibilities are in the host buffers.  Output always overwrites.  Uses
- * the channel-major path (corr_path 3 or 4 selects the correlator feed). */
+ * the corner turn and correlator of the context's corr_path (1, 2: as 4). */
 int dsax_correlate_many(dsax_ctx *ctx, const void *const *blocks, void *const *vis, int nblk,
                         int mem);
 
