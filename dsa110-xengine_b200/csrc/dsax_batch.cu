@@ -126,7 +126,7 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
   const size_t nscr = (size_t)maxch * cf.npkt * 256;
   const size_t nfb = (size_t)cf.nbeam * nout * (maxch / 8);
   const size_t nfs = 4 * (size_t)cf.nbeam * (maxch / 8) + (size_t)cf.nbeam * nout + 64 +
-                     (size_t)cf.nbeam * nout + flag_ctr_ints(cf.nbeam);
+                     (size_t)cf.nbeam * nout + flag_ctr_ints(cf.nbeam, maxch / 8);
   int rc;
   if ((rc = ensure_buffer(c, c->aux[AUX_BATCH_SCRATCH], nscr + 4 * (nfb + nfs), "batch scratch")) !=
       DSAX_OK)

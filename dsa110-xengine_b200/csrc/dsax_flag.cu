@@ -35,11 +35,11 @@ namespace dsax {
 
 namespace flag {
 constexpr int kStatThreads = 256;
-constexpr int kStages = 3;
-constexpr int kStageTarget = 24576;   // bytes per pipeline stage (upper bound)
+constexpr int kTargetCtas = 296;      // statistics CTAs below which time is chunked: two per SM
 constexpr int kMaxChan = 1024;
 constexpr int kApplyThreads = 256;    // apply / time-series CTA
 constexpr int kApplyRows = 256;       // rows per apply CTA
+constexpr int kApplyUnroll = 4;       // row groups of loads in flight
 constexpr int kMaxTsBase = 4096;
 constexpr int kLfMaxChan = 128;       // learned-flagger features: channels per beam
 constexpr int kDecThreads = 256;
@@ -108,67 +108,91 @@ __device__ void flag_decide_beam(const FlagArgs &a, int b, uint8_t *smem);
 __device__ void flag_total_power(const FlagArgs &a);
 
 // ---------------------------------------------------------------- statistics
-// One CTA per (channel slab of up to kFlagSlab channels, beam).  The slab's
-// rows stream through a three-stage ring of `rs` rows each (rs divides
-// TBIN), one 2-D TMA box [rs rows][min(nchan, 128) channels] per stage
-// (channels past nchan read zero), completing on the stage's mbarrier; the
-// waits are bounded (a.wait_limit_ns, recorded in a.err).  Every thread
-// fences its generic reads of a stage before the barrier after which the
-// stage is loaded again.  Thread (p, g) owns channels 4g..4g+3 of the slab and rows
-// p, p + P, ... of every stage (the lanes of a warp cover consecutive
-// 16-byte pieces of a row: conflict-free shared reads, coalesced global
-// writes); sums are FP64 for FP32 data and 32-bit integers for uint8 (at
-// most 32768 rows per thread, so 255^2 products stay below 2^31; the
-// launcher checks it), finished in shared memory in a fixed order (four
-// interleaved partial sums per reduction), so results do not depend on
-// scheduling.  With a scaley
-// baseline the stage is normalised in shared memory first and written back
-// (the statistics then describe the normalised block, as in the reference).
-// Per row the slab's raw sum goes to rowsum (or to ts when there is one
-// slab); flag_apply_kernel turns it into the channel-mean series after the
-// flagged columns are replaced.
-template <typename E>
+// One CTA per (channel slab of up to kFlagSlab channels, time chunk, beam).
+// A warp takes whole TBIN bins of the chunk (every eighth one), or, where the
+// chunk has fewer than eight, an eighth of each.  Its rows come as TMA boxes
+// of kBatch passes ([rows][min(nchan, 128) channels], channels past nchan
+// zero) into a ring of its own, a.ring - 1 boxes ahead, on its own mbarriers
+// (bounded waits, a.wait_limit_ns, recorded in a.err); a pass is as many
+// consecutive rows as the lanes hold 4-channel groups of.  So no warp waits
+// for another one in the loop.  (Stages for the whole CTA with two block
+// barriers and a partly idle row reduction each: 82 against 63 us for
+// [256][4096][48] FP32, of which some 26 are what a call costs at any length;
+// loads straight into registers: 94.  Scaled uint8 [64][16384][1024]: 1,138
+// against 700.)  What bounds it: the loop runs near the HBM rate for FP32; for
+// uint8 the 128-byte slab rows in and out (about 3.6 TB/s), in 1.7 waves of
+// CTAs.
+//
+// Sums are FP64 for FP32 data and exact 32-bit integers for uint8 (a lane
+// takes at most a quarter of the rows, so 255^2 products stay below 2^32; the
+// launcher checks it).  Four rows of uint8 are transposed to words of one
+// channel, whose sum and sum of squares are one dp4a each.  A lane's sums are
+// combined with the other row phases' in a fixed order, and the chunks' by the
+// chunk CTA that finishes last, in chunk order, so results do not depend on
+// scheduling.  With a scaley baseline each value is normalised as it is read
+// and written back (the statistics then describe the normalised block, as in
+// the reference).  Per row the slab's raw sum goes to rowsum (or to ts when
+// there is one slab): the lanes' partial sums of a batch of rows meet in the
+// warp's own shared buffer.  flag_apply_kernel turns it into the channel-mean
+// series after the flagged columns are replaced.
+namespace flag {
+constexpr int kWarps = kStatThreads / 32;
+template <typename E> constexpr int batch() { return std::is_same<E, float>::value ? 8 : 16; }
+constexpr int kMaxRing = 4;      // boxes of a warp's ring
+constexpr int kPartFields = 5;   // per channel of a chunk: sum, squares, max, bin max, bin min
+}  // namespace flag
+
+// kPix: also forms the downsampled spectrogram.  kG: the slab's 4-channel
+// groups where they are known when compiling (12, the 48 channel groups of a
+// subband; 32, a full slab), so that row and table strides are constants: a
+// third of the instructions of the general form (0).
+template <typename E, bool kPix, int kG>
 __global__ void __launch_bounds__(flag::kStatThreads, 2)
     flag_stats_kernel(const __grid_constant__ CUtensorMap tmap, FlagArgs a) {
-  constexpr int S = flag::kStages;
-  constexpr int ES = (int)sizeof(E);
-  const int slab = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-  const int T = a.ntime, C = a.nchan, TB = a.tbin, RS = a.rs;
+  constexpr bool kU8 = std::is_same<E, uint8_t>::value;
+  constexpr int kBatch = flag::batch<E>();
+  constexpr int kWarps = flag::kWarps;
+  constexpr bool kRedux = kU8 && kG == 32;     // a warp's pass is one row: warp-wide integer sums
+  using Acc = typename std::conditional<kU8, uint32_t, double>::type;   // sums of a lane
+  using Vec = typename std::conditional<kU8, uint32_t, float4>::type;   // four channels of a row
+  const int slab = (int)blockIdx.x % a.nslab, chunk = (int)blockIdx.x / a.nslab, b = blockIdx.y;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int T = a.ntime, C = a.nchan, TB = a.tbin;
   const int c0 = slab * kFlagSlab;
-  const int cs = min(kFlagSlab, C - c0);
-  const int G4 = cs >> 2, P = flag::kStatThreads / G4;
-  const int p = tid / G4, g = tid - p * G4;
-  const bool active = p < P;
-  const int nbins = T / TB, spb = TB / RS, nst = nbins * spb;
-  const int bx = C < kFlagSlab ? C : kFlagSlab;   // channels of a TMA box row
-  const int rb = bx * ES;                        // bytes of one staged row (multiple of 16)
-  const int stage_bytes = (RS * rb + 127) & ~127;
-  const int64_t rstride = (int64_t)C * ES;
-  const uint8_t *xb =
-      reinterpret_cast<const uint8_t *>(elem_in<E>(a) + (int64_t)b * T * C + c0);
+  const int cs = kG ? 4 * kG : min(kFlagSlab, C - c0);
+  const int G4 = kG ? kG : cs >> 2;
+  const int bx = kG ? 4 * kG : min(kFlagSlab, C);   // channels of a box row
+  const int rpw = 32 / (bx / 4);               // rows of a pass
+  // lanes past the last whole row repeat row phase 0 (the same values to the
+  // same places); `active` lanes give the totals
+  const bool active = lane < rpw * G4;
+  const int rp = active ? lane / G4 : 0, g = active ? lane - rp * G4 : lane % G4;
+  const bool lead = lane < G4;                 // row phase 0
+  const int nbins = T / TB;
+  const int bin0 = (int)((int64_t)nbins * chunk / a.nchunk);
+  const int bin1 = (int)((int64_t)nbins * (chunk + 1) / a.nchunk);
   E *xw = elem_out<E>(a);
   const bool scale = a.spec0 != nullptr;
+  E *const xo = (scale && xw) ? xw + (int64_t)b * T * C + c0 + 4 * g : nullptr;
 
-  constexpr bool kU8 = std::is_same<E, uint8_t>::value;
-  // row partials: exact ints for uint8, doubles for FP32
-  using RsT = typename std::conditional<kU8, int, double>::type;
   extern __shared__ __align__(128) uint8_t fs_raw[];
-  __shared__ __align__(8) uint64_t sfull[S];
+  __shared__ __align__(8) uint64_t sfull[kWarps][flag::kMaxRing];
   __shared__ volatile int sabort;
-  if (tid == 0) {
-    for (int s2 = 0; s2 < S; ++s2) mbar_init(&sfull[s2], 1);
-    sabort = 0;
-    mbar_fence_init();
-  }
-  const uint32_t sbase = smem_u32(fs_raw);
-  const int GS = G4 | 1;   // odd row stride: the row sums read column-wise conflict-free
-  RsT *sm_rs = reinterpret_cast<RsT *>(fs_raw + S * stage_bytes);         // [RS][GS]
-  double *sm_bp = reinterpret_cast<double *>(
-      fs_raw + S * stage_bytes + ((sizeof(RsT) * RS * GS + 15) & ~(size_t)15));   // [P][cs]
-  double *sm_k = sm_bp + P * cs;                                           // [cs]
-  float *sm_s0 = reinterpret_cast<float *>(sm_k + cs);                     // [cs]
-  float *sm_k2 = sm_s0 + cs;                                               // [cs] float(2k)
-  uint8_t *sm_lut = reinterpret_cast<uint8_t *>(sm_k2 + cs);               // uint8: [256][cs]
+  const int GS = G4 | 1;                       // odd row stride of the row buffer
+  const int brows = kBatch * rpw;              // rows of a batch
+  const int rb = bx * (int)sizeof(E);          // bytes of a staged row
+  const int stage_bytes = (brows * rb + 127) & ~127;
+  uint8_t *const ring = fs_raw + warp * a.ring * stage_bytes;   // the warp's stages
+  uint8_t *const fs_x = fs_raw + kWarps * a.ring * stage_bytes;
+  const int rstride = flag_rowbuf(cs, kBatch, rpw, (int)sizeof(Acc));
+  Acc *const rbuf = reinterpret_cast<Acc *>(fs_x + warp * rstride);
+  double *const sm_part = reinterpret_cast<double *>(fs_x);     // after the loop: [8 rpw][cs]
+  // per warp and channel: bin maximum and minimum (bin sums)
+  Acc *const sm_bx = reinterpret_cast<Acc *>(fs_x + kWarps * rstride);   // [8][2][cs]
+  double *const sm_k = reinterpret_cast<double *>(sm_bx + 2 * kWarps * cs);  // [cs]
+  float *const sm_s0 = reinterpret_cast<float *>(sm_k + cs);              // [cs]
+  float *const sm_k2 = sm_s0 + cs;                                        // [cs] float(2k)
+  uint8_t *const sm_lut = reinterpret_cast<uint8_t *>(sm_k2 + cs);        // uint8: [256][cs]
   const double inv_tb = 1.0 / TB;
 
   if (scale) {
@@ -177,42 +201,72 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
       sm_k[c] = (double)a.sig / (double)sqrtf(a.var0[b * C + c0 + c]);
       sm_k2[c] = (float)(2.0 * sm_k[c]);
     }
+    __syncthreads();
     if constexpr (kU8) {
       // uint8 has 256 inputs per channel: scaley as a table [x][channel],
       // read by the lanes of a warp (consecutive channel groups) from
       // distinct banks
-      __syncthreads();
       for (int i = tid; i < 256 * cs; i += flag::kStatThreads) {
         const int x = i / cs, c = i - x * cs;
         sm_lut[i] = (uint8_t)scaley_u8((float)x, sm_s0[c], sm_k2[c], sm_k[c], a.mn);
       }
     }
   }
+  for (int c = lane; c < cs; c += 32) {
+    sm_bx[(2 * warp) * cs + c] = kU8 ? (Acc)0 : (Acc)-1e300;
+    sm_bx[(2 * warp + 1) * cs + c] = kU8 ? (Acc)0xFFFFFFFFu : (Acc)1e300;
+  }
+  if (tid == 0) {
+    for (int w = 0; w < kWarps; ++w)
+      for (int i = 0; i < a.ring; ++i) mbar_init(&sfull[w][i], 1);
+    sabort = 0;
+    mbar_fence_init();
+  }
   __syncthreads();
-  // sum of n values at v[0], v[stride], ... in four interleaved chains
-  auto sum4 = [](const auto *v, int n, int stride) -> double {
-    using V = typename std::remove_cv<typename std::remove_pointer<decltype(v)>::type>::type;
-    V a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    int k = 0;
-    for (; k + 4 <= n; k += 4) {
-      a0 += v[k * stride];
-      a1 += v[(k + 1) * stride];
-      a2 += v[(k + 2) * stride];
-      a3 += v[(k + 3) * stride];
-    }
-    for (; k < n; ++k) a0 += v[k * stride];
-    return (double)((a0 + a1) + (a2 + a3));
-  };
 
-  // stage st: one TMA box, issued by thread 0
-  const uint32_t box_bytes = (uint32_t)(RS * rb);
-  int issued = 0;
-  auto issue = [&](int st) {
-    if (st < nst) {
-      mbar_arrive_expect_tx(&sfull[st % S], box_bytes);
-      tma_load_2d(sbase + (uint32_t)(st % S) * stage_bytes, &tmap, c0, b * T + st * RS,
-                  &sfull[st % S]);
-      issued = st + 1;
+  Acc s[4], q[4], bs[4];                       // sums, squares, sums of the current bin
+  float m[4];                                  // maxima (uint8: in mx)
+  uint32_t mx[2] = {0u, 0u};                   // uint8 maxima of channels 0, 2 and 1, 3
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    s[j] = 0; q[j] = 0; bs[j] = 0;
+    m[j] = -INFINITY;
+  }
+  // the running pixel of channels lane, lane + 32, ... (sum and maximum over
+  // tds rows in row order, FP32), and its rows so far
+  constexpr int kPixC = kFlagSlab / 32;
+  float px_s[kPixC], px_m[kPixC];
+  int px_n = 0;
+#pragma unroll
+  for (int k = 0; k < kPixC; ++k) {
+    px_s[k] = 0.0f;
+    px_m[k] = -INFINITY;
+  }
+
+  // scaley of four channels by the table (one extraction, one multiply-add
+  // and one load per sample: explicit shared addresses keep it at that)
+  const uint32_t lut_base = smem_u32(sm_lut) + 4u * g;
+  auto lut4 = [&](uint32_t w) -> uint32_t {
+    uint32_t y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      asm("ld.shared.u8 %0, [%1];" : "=r"(y[j]) : "r"(__byte_perm(w, 0u, 0x4440u + j) * cs + lut_base + j));
+    return __byte_perm(__byte_perm(y[0], y[1], 0x0040u), __byte_perm(y[2], y[3], 0x0040u), 0x5410u);
+  };
+  auto take_u8 = [&](const uint32_t (&w)[4]) {
+    const uint32_t t0 = __byte_perm(w[0], w[1], 0x5140u), t1 = __byte_perm(w[0], w[1], 0x7362u);
+    const uint32_t t2 = __byte_perm(w[2], w[3], 0x5140u), t3 = __byte_perm(w[2], w[3], 0x7362u);
+    const uint32_t x[4] = {__byte_perm(t0, t2, 0x5410u), __byte_perm(t0, t2, 0x7632u),
+                           __byte_perm(t1, t3, 0x5410u), __byte_perm(t1, t3, 0x7632u)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      bs[j] = (Acc)__dp4a(x[j], 0x01010101u, (uint32_t)bs[j]);
+      q[j] = (Acc)__dp4a(x[j], x[j], (uint32_t)q[j]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+      mx[0] = __vimax3_u16x2(mx[0], w[k] & 0x00FF00FFu, w[k + 1] & 0x00FF00FFu);
+      mx[1] = __vimax3_u16x2(mx[1], (w[k] >> 8) & 0x00FF00FFu, (w[k + 1] >> 8) & 0x00FF00FFu);
     }
   };
   auto put_row = [&](int t, double r) {
@@ -221,186 +275,337 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
     else
       a.rowsum[((int64_t)b * a.nslab + slab) * T + t] = (float)r;
   };
-  // normalise (if scaling) and accumulate the four channels of one row:
-  // FP64 for FP32 data, exact 32-bit integers for uint8 (no FP64 work)
-  using Acc = typename std::conditional<kU8, int, double>::type;
-  using MaxT = typename std::conditional<kU8, int, float>::type;
-  Acc s[4], q[4], bs[4];
-  MaxT m[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    s[j] = 0; q[j] = 0; bs[j] = 0;
-    m[j] = kU8 ? (MaxT)0 : (MaxT)-INFINITY;
-  }
-  auto take = [&](uint8_t *src, int t, bool bin, bool keep) -> RsT {
-    float v[4];
+  // one batch of rows from t on, the first `n` of them (kWhole: all brows)
+  auto batch = [&](auto whole_t, const uint8_t *sp, int t, int n) {
+    constexpr bool kWhole = decltype(whole_t)::value;
+    const uint32_t src = smem_u32(sp) + rp * rb + g * (int)sizeof(Vec);
+    [[maybe_unused]] Acc *const rs = rbuf + rp * GS + g;
+    // (uint8: at most 2^28 samples of a beam, so 32-bit offsets)
+    using Off = typename std::conditional<kU8, uint32_t, int64_t>::type;
+    E *const dst = xo;
+    const Off doff = (Off)(t + rp) * (Off)C, step = (Off)rpw * (Off)C;
+    [[maybe_unused]] uint32_t rsum[kBatch / 2];   // full uint8 slabs: row sums of two rows each
     if constexpr (kU8) {
-      uint32_t w = *reinterpret_cast<const uint32_t *>(src);
-      if (scale) {
-        uint32_t o = 0u;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          o |= (uint32_t)sm_lut[((w >> (8 * j)) & 255u) * cs + 4 * g + j] << (8 * j);
-        w = o;
-        if (xw) *reinterpret_cast<uint32_t *>(xw + ((int64_t)b * T + t) * C + c0 + 4 * g) = w;
-      }
+      for (int u = 0; u < kBatch; u += 4) {
+        uint32_t w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int x = (int)((w >> (8 * j)) & 255u);
-        if (bin) bs[j] += x; else s[j] += x;
-        q[j] += x * x;
-        m[j] = max(m[j], x);
+        for (int i = 0; i < 4; ++i)
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(src + (u + i) * rpw * rb));
+        if (scale) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w[i] = lut4(w[i]);
+        }
+        if constexpr (!kWhole) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (rp + (u + i) * rpw >= n) w[i] = 0u;
+        }
+        if (dst) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (kWhole || rp + (u + i) * rpw < n)
+              __stcs(reinterpret_cast<uint32_t *>(dst + (doff + (u + i) * step)), w[i]);
+        }
+        if constexpr (kRedux) {   // a row of at most 128 x 255 fits 16 bits
+#pragma unroll
+          for (int i = 0; i < 4; i += 2)
+            rsum[(u + i) / 2] = __reduce_add_sync(
+                0xffffffffu, __dp4a(w[i], 0x01010101u, 0u) + (__dp4a(w[i + 1], 0x01010101u, 0u) << 16));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) rs[(u + i) * rpw * GS] = __dp4a(w[i], 0x01010101u, 0u);
+        }
+        take_u8(w);
       }
-      return (int)__dp4a(w, 0x01010101u, 0u);   // the row's four bytes summed
     } else {
-      ld4<E>(src, v);
-      if (scale) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          v[j] = scaley1<E>(v[j], sm_s0[4 * g + j], sm_k[4 * g + j], a.mn);
-        if (xw) st4<E>(xw + ((int64_t)b * T + t) * C + c0 + 4 * g, v);
-        if (keep) st4<E>(src, v);   // the pixel sums read the normalised stage
-      }
-      double r = 0.0;
+      for (int u = 0; u < kBatch; ++u) {
+        if (kWhole || rp + u * rpw < n) {
+          float x[4];
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                       : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(src + u * rpw * rb));
+          if (scale) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (bin) bs[j] += v[j]; else s[j] += v[j];
-        q[j] += (double)v[j] * v[j];
-        m[j] = fmaxf(m[j], v[j]);
-        r += v[j];
+            for (int j = 0; j < 4; ++j) x[j] = scaley1<E>(x[j], sm_s0[4 * g + j], sm_k[4 * g + j], a.mn);
+            if (dst) st4<E>(dst + (doff + u * step), x);
+          }
+          const double d0 = (double)x[0], d1 = (double)x[1], d2 = (double)x[2], d3 = (double)x[3];
+          bs[0] += d0; bs[1] += d1; bs[2] += d2; bs[3] += d3;
+          q[0] += d0 * d0; q[1] += d1 * d1; q[2] += d2 * d2; q[3] += d3 * d3;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], x[j]);
+          rs[u * rpw * GS] = ((d0 + d1) + d2) + d3;
+        }
       }
-      return r;
+    }
+    if constexpr (kPix) {   // from the staged rows (whole pixels per range of rows)
+      const float *sf = reinterpret_cast<const float *>(sp);
+      const int nr = kWhole ? brows : n;
+#pragma unroll 1
+      for (int r0 = 0; r0 < nr;) {
+        const int r1 = min(nr, r0 + a.tds - px_n);
+        px_n += r1 - r0;
+#pragma unroll 4
+        for (int r = r0; r < r1; ++r)
+#pragma unroll
+          for (int k = 0; k < kPixC; ++k)
+            if (lane + 32 * k < cs) {
+              const float v = sf[r * bx + lane + 32 * k];
+              px_s[k] += v;
+              px_m[k] = fmaxf(px_m[k], v);
+            }
+        r0 = r1;
+        if (px_n < a.tds) break;
+        px_n = 0;
+        const int64_t o = ((int64_t)b * (T / a.tds) + (t + r1) / a.tds - 1) * C + c0;
+#pragma unroll
+        for (int k = 0; k < kPixC; ++k)
+          if (lane + 32 * k < cs) {
+            a.pix_sum[o + lane + 32 * k] = px_s[k];
+            a.pix_max[o + lane + 32 * k] = px_m[k];
+            px_s[k] = 0.0f;
+            px_m[k] = -INFINITY;
+          }
+      }
+    }
+    if constexpr (kRedux) {   // lane k keeps and writes the sum of row k
+      uint32_t v = 0u;
+#pragma unroll
+      for (int k = 0; k < kBatch / 2; ++k)
+        if ((lane >> 1) == k) v = rsum[k];
+      if (lane < (kWhole ? kBatch : n)) put_row(t + lane, (double)((lane & 1) ? v >> 16 : v & 0xFFFFu));
+      return;
+    }
+    __syncwarp();
+    // row sums: lr lanes per row, then a shuffle tree (batches of 8 or 16 rows
+    // fill the warp exactly; larger ones take one lane per row)
+    static_assert(kBatch == 8 || kBatch == 16, "every lane takes part in the row shuffles");
+    const int lr = brows <= 8 ? 4 : brows <= 16 ? 2 : 1;
+    const int sub = lane & (lr - 1);
+    for (int k = lane / lr; k < brows; k += 32 / lr) {
+      const Acc *w = rbuf + k * GS;
+      Acc a0 = 0, a1 = 0;
+      int e = sub;
+      for (; e + lr < G4; e += 2 * lr) {
+        a0 += w[e];
+        a1 += w[e + lr];
+      }
+      if (e < G4) a0 += w[e];
+      a0 += a1;
+      for (int o = 1; o < lr; o <<= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      if (sub == 0 && (kWhole || k < n)) put_row(t + k, (double)a0);
+    }
+    __syncwarp();
+  };
+  // `count` ranges of n rows, tstep apart from t0 on: boxes of brows rows (the
+  // last of a range may reach past it), a.ring - 1 ahead through all of the
+  // ranges, taken one after the other; `end` after each range
+  uint32_t is = 0, cs_i = 0, cs_ph = 0;        // ring positions: issue, consume (and its parity)
+  auto run = [&](int t0, int n, int tstep, int count, auto end) {
+    int ir = 0, ik = 0;                        // next box to issue
+    auto issue = [&]() {
+      if (ir >= count || n <= 0) return;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&sfull[warp][is], (uint32_t)(brows * rb));
+        tma_load_2d(smem_u32(ring) + is * stage_bytes, &tmap, c0, b * T + t0 + ir * tstep + ik,
+                    &sfull[warp][is]);
+      }
+      if (++is == (uint32_t)a.ring) is = 0;
+      ik += brows;
+      if (ik >= n) {
+        ik = 0;
+        ++ir;
+      }
+    };
+    for (int i = 0; i + 1 < a.ring; ++i) issue();
+#pragma unroll 1
+    for (int r = 0; r < count; ++r) {
+#pragma unroll 1
+      for (int k0 = 0; k0 < n; k0 += brows) {
+        issue();
+        const bool ok = mbar_wait_bounded(&sfull[warp][cs_i], cs_ph, &sabort, a.err, DEV_ERR_WAIT_FULL,
+                                          a.wait_limit_ns);
+        if (!__all_sync(0xffffffffu, ok)) {    // recorded in a.err; the box lands before the CTA exits
+          volatile int no_abort = 0;
+          mbar_wait_bounded(&sfull[warp][cs_i], cs_ph, &no_abort, a.err, DEV_ERR_WAIT_FULL,
+                            drain_limit(a.wait_limit_ns));
+        } else {
+          const uint8_t *sp = ring + cs_i * stage_bytes;
+          const int t = t0 + r * tstep + k0;
+          if (k0 + brows <= n) batch(std::true_type{}, sp, t, brows);
+          else batch(std::false_type{}, sp, t, n - k0);
+        }
+        // the stage's reads before the box that overwrites it
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (++cs_i == (uint32_t)a.ring) {
+          cs_i = 0;
+          cs_ph ^= 1u;
+        }
+      }
+      end();
     }
   };
-  double bmax = -1e300, bmin = 1e300;   // owned by thread tid < cs (channel tid)
-
-  if (tid == 0)
-    for (int i = 0; i < S - 1; ++i) issue(i);
-  int consumed = 0;
-  for (int st = 0; st < nst; ++st) {
-    if (tid == 0) issue(st + S - 1);   // its slot was released at the end of stage st - 1
-    const bool ok = mbar_wait_bounded(&sfull[st % S], (uint32_t)(st / S) & 1u, &sabort, a.err,
-                                      DEV_ERR_WAIT_FULL, a.wait_limit_ns);
-    if (__syncthreads_or(!ok)) break;
-    consumed = st + 1;
-    uint8_t *sp = fs_raw + (st % S) * stage_bytes;
-    const int t0 = st * RS;
-    if (active) {
-      for (int r = p; r < RS; r += P) {
-        sm_rs[r * GS + g] = take(sp + r * rb + 4 * g * ES, t0 + r, true, a.pix_sum != nullptr);
-      }
-    }
-    const bool bin_end = (st + 1) % spb == 0;
-    if (spb == 1 && active) {   // one stage per bin: its partials go out with the rows
+  // the bin's sums over the row phases -> its extremes (phase 0's lanes)
+  auto bin_total = [&](int j) -> Acc {
+    Acc t = bs[j];
+    for (int k = 1; k < rpw; ++k) t += __shfl_sync(0xffffffffu, bs[j], (lane + k * G4) & 31);
+    return t;
+  };
+  if (bin1 - bin0 >= kWarps) {
+    run((bin0 + warp) * TB, TB, kWarps * TB, (bin1 - bin0 - warp + kWarps - 1) / kWarps, [&]() {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        sm_bp[p * cs + 4 * g + j] = (double)bs[j];
+        const Acc t = bin_total(j);
+        if (lead) {
+          Acc *e = sm_bx + 2 * warp * cs + 4 * g + j;
+          e[0] = max(e[0], t);
+          e[cs] = min(e[cs], t);
+        }
         s[j] += bs[j];
         bs[j] = 0;
       }
-    }
-    if (a.pix_sum) {   // downsampled spectrogram: rs / tds whole pixel rows per stage
-      __syncthreads();
-      const float *sf = reinterpret_cast<const float *>(sp);
-      const int npr = RS / a.tds, H = T / a.tds;
-      for (int i = tid; i < npr * cs; i += flag::kStatThreads) {
-        const int pr = i / cs, c = i - pr * cs;
-        float sum = 0.f, mx = -INFINITY;
-        for (int r = 0; r < a.tds; ++r) {
-          const float v = sf[(pr * a.tds + r) * cs + c];
-          sum += v;
-          mx = fmaxf(mx, v);
-        }
-        const int64_t o = ((int64_t)b * H + t0 / a.tds + pr) * C + c0 + c;
-        a.pix_sum[o] = sum;
-        a.pix_max[o] = mx;
-      }
-    }
-    fence_proxy_async_smem();   // this stage's generic reads before its next TMA write
-    __syncthreads();
-    if (tid < RS) put_row(t0 + tid, sum4(sm_rs + tid * GS, G4, 1));
-    if (bin_end) {   // the last stage of a TBIN bin: bin means per channel
-      if (spb > 1) {
-        if (active) {
+    });
+  } else {
+    // few bins: an eighth of the rows (in passes, or pixel rows) of each per
+    // warp, the bin's sums combined by the CTA
+    const int unit = kPix ? a.tds : rpw;
+    const int units = (TB + unit - 1) / unit, per = (units + kWarps - 1) / kWarps;
+#pragma unroll 1
+    for (int bin = bin0; bin < bin1; ++bin) {
+      const int r0 = min(TB, warp * per * unit), r1 = min(TB, (warp + 1) * per * unit);
+      run(bin * TB + r0, r1 - r0, 0, 1, []() {});
+      __syncthreads();   // the row buffers become [8][cs] partial bin sums
+      Acc *const bp = reinterpret_cast<Acc *>(fs_x);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            sm_bp[p * cs + 4 * g + j] = (double)bs[j];
-            s[j] += bs[j];
-            bs[j] = 0;
-          }
-        }
-        __syncthreads();
+      for (int j = 0; j < 4; ++j) {
+        const Acc t = bin_total(j);
+        if (lead) bp[warp * cs + 4 * g + j] = t;
+        s[j] += bs[j];
+        bs[j] = 0;
       }
-      if (tid < cs) {
-        const double mb = sum4(sm_bp + tid, P, cs) * inv_tb;
-        bmax = fmax(bmax, mb);
-        bmin = fmin(bmin, mb);
+      __syncthreads();
+      for (int c = tid; c < cs; c += flag::kStatThreads) {
+        Acc t = 0;
+        for (int w = 0; w < kWarps; ++w) t += bp[w * cs + c];
+        sm_bx[c] = max(sm_bx[c], t);
+        sm_bx[cs + c] = min(sm_bx[cs + c], t);
       }
+      __syncthreads();
     }
   }
-  // boxes still landing after an abort: wait for them before exit
-  if (tid == 0) {
-    volatile int no_abort = 0;
-    for (int k = consumed; k < issued; ++k)
-      mbar_wait_bounded(&sfull[k % S], (uint32_t)(k / S) & 1u, &no_abort, a.err, DEV_ERR_WAIT_FULL,
-                        drain_limit(a.wait_limit_ns));
+  // rows beyond the last whole bin: everything but the bins
+  if (chunk == a.nchunk - 1 && nbins * TB < T) {
+    const int n = T - nbins * TB, per = ((n + rpw - 1) / rpw + kWarps - 1) / kWarps * rpw;
+    const int r0 = min(n, warp * per), r1 = min(n, (warp + 1) * per);
+    run(nbins * TB + r0, r1 - r0, 0, 1, []() {});
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[j] += bs[j];
+      bs[j] = 0;
+    }
   }
   __syncthreads();
   if (sabort) return;   // recorded in a.err; no statistics from this CTA
-  // rows beyond the last whole bin (T % TB): sums, squares, max and row
-  // sums, read directly
-  for (int t0 = nbins * TB; t0 < T; t0 += RS) {
-    __syncthreads();
-    const int rows = min(RS, T - t0);
-    if (active) {
-      for (int r = p; r < rows; r += P)
-        sm_rs[r * GS + g] = take(const_cast<uint8_t *>(xb) + (int64_t)(t0 + r) * rstride + 4 * g * ES,
-                                 t0 + r, false, false);
-    }
-    __syncthreads();
-    if (tid < rows) put_row(t0 + tid, sum4(sm_rs + tid * GS, G4, 1));
-  }
-  // per-channel totals over the P row phases, in phase order
+  // per-channel totals over the row phases of every warp, in order
+  const int P = kWarps * rpw;
   double tot[3] = {0.0, 0.0, -INFINITY};
 #pragma unroll
   for (int pass = 0; pass < 3; ++pass) {
     __syncthreads();
     if (active) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        sm_bp[p * cs + 4 * g + j] =
-            pass == 0 ? (double)s[j] : pass == 1 ? (double)q[j] : (double)m[j];
+      for (int j = 0; j < 4; ++j) {
+        const double mj = kU8 ? (double)((mx[j & 1] >> (8 * (j & 2))) & 0xFFFFu) : (double)m[j];
+        sm_part[(warp * rpw + rp) * cs + 4 * g + j] = pass == 0 ? (double)s[j] : pass == 1 ? (double)q[j] : mj;
+      }
     }
     __syncthreads();
     if (tid < cs) {
       if (pass < 2) {
-        tot[pass] = sum4(sm_bp + tid, P, cs);
+        double a0 = 0.0, a1 = 0.0;
+        for (int k = 0; k + 1 < P; k += 2) {
+          a0 += sm_part[k * cs + tid];
+          a1 += sm_part[(k + 1) * cs + tid];
+        }
+        tot[pass] = a0 + a1;                   // (P is a multiple of 8)
       } else {
-        for (int k = 0; k < P; ++k) tot[2] = fmax(tot[2], sm_bp[k * cs + tid]);
+        for (int k = 0; k < P; ++k) tot[2] = fmax(tot[2], sm_part[k * cs + tid]);
       }
     }
   }
-  if (tid < cs) {
+  double bmax = -1e300, bmin = 1e300;          // bin sums
+  if (tid < cs && bin1 > bin0) {
+    Acc hi = sm_bx[tid], lo = sm_bx[cs + tid];
+    for (int w = 1; w < kWarps; ++w) {
+      hi = max(hi, sm_bx[2 * w * cs + tid]);
+      lo = min(lo, sm_bx[(2 * w + 1) * cs + tid]);
+    }
+    bmax = (double)hi;
+    bmin = (double)lo;
+  }
+  __shared__ int last_sh;
+  if (a.nchunk > 1) {
+    // the chunk's partial results; the (beam, slab)'s last chunk CTA combines
+    // them in chunk order (nothing waits)
+    double *const part = a.part + ((int64_t)b * a.nslab + slab) * a.nchunk * flag::kPartFields * kFlagSlab;
+    if (tid < cs) {
+      double *o = part + (int64_t)chunk * flag::kPartFields * kFlagSlab + tid;
+      o[0] = tot[0];
+      o[kFlagSlab] = tot[1];
+      o[2 * kFlagSlab] = tot[2];
+      o[3 * kFlagSlab] = bmax;
+      o[4 * kFlagSlab] = bmin;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0)
+      last_sh = atomicAdd(a.ctr + flag_ctr_chunk(a.nbeam) + b * a.nslab + slab, 1) == a.nchunk - 1;
+    __syncthreads();
+    if (!last_sh) {
+      if (!a.decide || (!a.modcheck && !a.tpwr_out)) return;
+    } else {
+      __threadfence();
+      if (tid < cs) {
+        tot[0] = tot[1] = 0.0;
+        tot[2] = -INFINITY;
+        bmax = -1e300;
+        bmin = 1e300;
+        for (int k = 0; k < a.nchunk; ++k) {
+          const double *o = part + (int64_t)k * flag::kPartFields * kFlagSlab + tid;
+          tot[0] += __ldcg(o);
+          tot[1] += __ldcg(o + kFlagSlab);
+          tot[2] = fmax(tot[2], __ldcg(o + 2 * kFlagSlab));
+          bmax = fmax(bmax, __ldcg(o + 3 * kFlagSlab));
+          bmin = fmin(bmin, __ldcg(o + 4 * kFlagSlab));
+        }
+      }
+    }
+  }
+  const bool owner = a.nchunk == 1 || last_sh;
+  if (owner && tid < cs) {
     const double mean = tot[0] / T;
     const double var = fmax(tot[1] / T - mean * mean, 0.0);
     const int o = b * C + c0 + tid;
     a.spec[o] = (float)mean;
     a.var[o] = (float)var;
     a.maxs[o] = a.parity ? (float)mean : (float)tot[2];
-    a.pp[o] = nbins > 0 ? (float)(bmax - bmin) : 0.0f;
+    a.pp[o] = nbins > 0 ? (float)(bmax * inv_tb - bmin * inv_tb) : 0.0f;
   }
   if (!a.decide) return;
   // The last slab CTA of the beam makes its channel decisions, and the last
   // CTA of the grid the block-level total power: each CTA publishes its
   // statistics (fence) before counting itself in; nothing waits.
-  __shared__ int last_sh;
   __threadfence();
   __syncthreads();
-  if (tid == 0) last_sh = a.nslab == 1 ? 1 : (atomicAdd(a.ctr + b, 1) == a.nslab - 1);
-  __syncthreads();
-  if (last_sh) {
-    __threadfence();
-    flag_decide_beam(a, b, fs_raw);
+  if (owner) {
+    if (tid == 0) last_sh = a.nslab == 1 ? 1 : (atomicAdd(a.ctr + b, 1) == a.nslab - 1);
+    __syncthreads();
+    if (last_sh) {
+      __threadfence();
+      flag_decide_beam(a, b, fs_raw);
+    }
   }
   if (!a.modcheck && !a.tpwr_out) return;
   __syncthreads();
@@ -424,8 +629,27 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+// Up to kRankMax values the element of rank k is found by counting instead (one
+// barrier for 16: of the 48 channels' decisions the four-pass select was half).
+constexpr int kRankMax = 128;
 __device__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist, uint32_t *sel,
                                   int gtid, int gsize, int bid) {
+  if (n <= kRankMax) {
+    for (int i = gtid; i < n; i += gsize) {
+      const uint32_t x = ordered_key(v[i]);
+      int r = 0;
+#pragma unroll 4
+      for (int q = 0; q < n; ++q) {
+        const uint32_t y = ordered_key(v[q]);
+        r += y < x || (y == x && q < i);
+      }
+      if (r == k) sel[0] = __float_as_uint(v[i]);
+    }
+    named_bar(bid, gsize);
+    const float out = __uint_as_float(sel[0]);
+    named_bar(bid, gsize);
+    return out;
+  }
   uint32_t prefix = 0u, pmask = 0u;
   int kk = k;
   for (int shift = 24; shift >= 0; shift -= 8) {
@@ -470,16 +694,51 @@ __device__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist, 
   return __uint_as_float(u);
 }
 
-// channflag (src/gpu_flagger.cu:655-720) for one beam in a group of `gsize`
-// threads: forward nFiltSize-channel median detrend, then |x| > Thr * MAD
-// of the detrended spectrum inside the guard band (compared against 0, as
-// the reference does).  Medians are lower medians (medval, :534-556).
-__device__ void grp_channflag(const float *sb, float thr, const FlagArgs &a, uint8_t *mask,
-                              float *corr, float *tmp, uint32_t *hist, uint32_t *sel, int gtid,
-                              int gsize, int bid) {
+// One window of channflag's detrend: v - lower median of x[0..kF), the median
+// by rank counting with ties by index, in registers (a thread per window;
+// with a thread per window element and shared loads it was 70 us of the 1,024
+// channels' decisions).  Nothing is written where no element has the rank
+// (NaN data).
+template <int kF>
+__device__ __forceinline__ void window_median(const float *x, float v, float *out) {
+  float e[kF];
+  int r[kF];
+#pragma unroll
+  for (int i = 0; i < kF; ++i) {
+    e[i] = x[i];
+    r[i] = 0;
+  }
+#pragma unroll
+  for (int i = 0; i < kF; ++i)
+#pragma unroll
+    for (int q = i + 1; q < kF; ++q) {
+      r[i] += e[q] < e[i];
+      r[q] += e[i] <= e[q];
+    }
+#pragma unroll
+  for (int i = 0; i < kF; ++i)
+    if (r[i] == (kF + 1) / 2 - 1) *out = v - e[i];
+}
+
+// The windows of channflag (src/gpu_flagger.cu:655-720) of the three spectra at
+// sb0, sb0 + 3 C and sb0 + 6 C, each detrended into its next C floats: forward
+// nFiltSize-channel median detrend inside the guard band, by `gsize` threads.
+__device__ void grp_detrend3(float *sb0, const FlagArgs &a, int gtid, int gsize) {
   const int C = a.nchan, G = a.guard, F = a.filt, n = C - 2 * G;
   const int kf = (F + 1) / 2 - 1;
-  for (int idx = gtid; idx < n * F; idx += gsize) {   // forward median detrend
+  if (F == 21) {   // nFiltSize
+    for (int id = gtid; id < 3 * n; id += gsize) {
+      const int k = id / n, jj = id - k * n;
+      float *sb = sb0 + 3 * C * k;
+      const int j = G + jj, w0 = (C - G - j >= F) ? j : C - G - F;
+      window_median<21>(sb + w0, sb[j], sb + C + jj);
+    }
+    return;
+  }
+  for (int id = gtid; id < 3 * n * F; id += gsize) {
+    const int k = id / (n * F), idx = id - k * n * F;
+    const float *sb = sb0 + 3 * C * k;
+    float *corr = sb0 + 3 * C * k + C;
     const int jj = idx / F, i = idx - jj * F;
     const int j = G + jj;
     const int w0 = (C - G - j >= F) ? j : C - G - F;
@@ -491,7 +750,15 @@ __device__ void grp_channflag(const float *sb, float thr, const FlagArgs &a, uin
     }
     if (r == kf) corr[jj] = sb[j] - x;
   }
-  named_bar(bid, gsize);
+}
+
+// channflag's decisions from the detrended spectrum: |x| > Thr * MAD inside
+// the guard band (compared against 0, as the reference does).  Medians are
+// lower medians (medval, :534-556).
+__device__ void grp_channflag(float thr, const FlagArgs &a, uint8_t *mask, const float *corr,
+                              float *tmp, uint32_t *hist, uint32_t *sel, int gtid, int gsize,
+                              int bid) {
+  const int C = a.nchan, G = a.guard, n = C - 2 * G;
   const int k = (n + 1) / 2 - 1;
   const float med = grp_radix_select(corr, n, k, hist, sel, gtid, gsize, bid);
   for (int i = gtid; i < n; i += gsize) tmp[i] = fabsf(corr[i] - med);
@@ -523,10 +790,13 @@ __device__ void flag_decide_beam(const FlagArgs &a, int b, uint8_t *smem) {
   const float *src = g == 0 ? a.spec : g == 1 ? a.var : g == 2 ? a.maxs : a.pp;
   for (int c = gtid; c < C; c += gsize)
     sb[c] = src[b * C + c] - ((g == 0 && a.oldspec) ? a.oldspec[b * C + c] : 0.0f);
-  named_bar(bid, gsize);
+  __syncthreads();
+  // the three detrends by the whole CTA, then a test per group
+  grp_detrend3(dsh, a, tid, flag::kStatThreads);
+  __syncthreads();
   if (g < 3) {
     const float thr = g == 1 ? a.thresh + a.var_add : a.thresh;
-    grp_channflag(sb, thr, a, cmask, corr, tm, hist[g], sel[g], gtid, gsize, bid);
+    grp_channflag(thr, a, cmask, corr, tm, hist[g], sel[g], gtid, gsize, bid);
   } else {   // simple_channflag (:559-610)
     for (int i = gtid; i < n; i += gsize) corr[i] = sb[G + i];
     named_bar(bid, gsize);
@@ -567,7 +837,18 @@ __device__ void flag_total_power(const FlagArgs &a) {
   __shared__ double red[flag::kStatThreads];
   const int tid = threadIdx.x, BC = a.nbeam * a.nchan;
   double acc = 0.0;
-  for (int i = tid; i < BC; i += flag::kStatThreads) acc += a.spec[i];
+  // (in order; the loads of 16 values are in flight together)
+  for (int i0 = tid; i0 < BC; i0 += 16 * flag::kStatThreads) {
+    float v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int i = i0 + k * flag::kStatThreads;
+      v[k] = i < BC ? __ldcg(a.spec + i) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      if (i0 + k * flag::kStatThreads < BC) acc += v[k];
+  }
   red[tid] = acc;
   __syncthreads();
   if (tid == 0) {
@@ -659,6 +940,7 @@ __global__ void __launch_bounds__(flag::kApplyThreads) flag_apply_kernel(FlagArg
     if (lane == 0) nact_sh = base;
   }
   __syncthreads();
+  __shared__ double corr_sh[flag::kApplyRows];   // per row: sum over flagged channels of (level - x)
   const int nact = nact_sh;
   const E re = repl_elem<E>(lev_sh);
   const float rf = (float)re;
@@ -666,38 +948,82 @@ __global__ void __launch_bounds__(flag::kApplyThreads) flag_apply_kernel(FlagArg
   while (L < nact && L < 32) L <<= 1;
   const int rpw = 32 / L, sub = lane & (L - 1);
   const E *xin = (a.spec0 && elem_out<E>(a)) ? elem_out<E>(a) : elem_in<E>(a);
-  for (int r0 = t_begin + warp * rpw; r0 < t_end; r0 += nw * rpw) {   // uniform per warp
-    const int t = r0 + lane / L;
-    double corr = 0.0;
-    if (t < t_end) {
-      const uint4 *row = reinterpret_cast<const uint4 *>(xin + ((int64_t)b * T + t) * C);
-      uint4 *wrow = xw ? reinterpret_cast<uint4 *>(xw + ((int64_t)b * T + t) * C) : nullptr;
-      for (int i = sub; i < nact; i += L) {
-        const uint32_t ce = chk[i];
-        const int k = (int)(ce & 0xFFFFu);
-        const uint32_t m = ce >> 16;
-        uint4 v = row[k];
-        E *ve = reinterpret_cast<E *>(&v);
+  for (int i = tid; i < flag::kApplyRows; i += flag::kApplyThreads) corr_sh[i] = 0.0;
+  __syncthreads();
+  // a lane keeps one chunk (and its element masks) while its warp goes down
+  // the rows, kApplyUnroll row groups of loads in flight
+  const int64_t rowlen = C / EPC;              // 16-byte words
+  const uint4 *xrow = reinterpret_cast<const uint4 *>(xin + (int64_t)b * T * C);
+  uint4 *wrow = xw ? reinterpret_cast<uint4 *>(xw + (int64_t)b * T * C) : nullptr;
+  for (int i0 = 0; i0 < nact; i0 += L) {
+    const bool have = i0 + sub < nact;
+    const uint32_t ce = have ? chk[i0 + sub] : 0u;
+    const int k = (int)(ce & 0xFFFFu);
+    const uint32_t m = ce >> 16;
+    uint32_t mk[4];                            // bit masks of the flagged elements, per word
 #pragma unroll
-        for (int e = 0; e < EPC; ++e)
-          if ((m >> e) & 1u) {
-            corr += (double)(rf - (float)ve[e]);
-            ve[e] = re;
-          }
-        if (wrow) wrow[k] = v;
-      }
-    }
-    for (int o = L >> 1; o > 0; o >>= 1) corr += __shfl_xor_sync(0xffffffffu, corr, o);
-    if (t < t_end && sub == 0) {
-      double rsum;
-      if (a.nslab == 1) {
-        rsum = a.ts[(int64_t)b * T + t];
+    for (int w = 0; w < 4; ++w) {
+      if constexpr (ES == 4) {
+        mk[w] = (m >> w) & 1u ? 0xFFFFFFFFu : 0u;
       } else {
-        rsum = 0.0;
-        for (int s = 0; s < a.nslab; ++s) rsum += a.rowsum[((int64_t)b * a.nslab + s) * T + t];
+        const uint32_t n4 = (m >> (4 * w)) & 15u;
+        mk[w] = (((n4 & 1u) | ((n4 & 2u) << 7) | ((n4 & 4u) << 14) | ((n4 & 8u) << 21)) * 255u);
       }
-      a.ts[(int64_t)b * T + t] = (float)((rsum + corr) / C);
     }
+    uint32_t rw;                               // the level in every element of a word
+    if constexpr (ES == 4) rw = __float_as_uint(re); else rw = (uint32_t)re * 0x01010101u;
+    for (int r0 = t_begin + warp * rpw; r0 < t_end; r0 += flag::kApplyUnroll * nw * rpw) {   // uniform
+      uint4 v[flag::kApplyUnroll];
+#pragma unroll
+      for (int u = 0; u < flag::kApplyUnroll; ++u) {
+        const int t = r0 + u * nw * rpw + lane / L;
+        if (have && t < t_end) v[u] = xrow[(int64_t)t * rowlen + k];
+      }
+#pragma unroll
+      for (int u = 0; u < flag::kApplyUnroll; ++u) {
+        const int t = r0 + u * nw * rpw + lane / L;
+        const bool on = have && t < t_end;
+        uint32_t x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        double corr = 0.0;
+        if (on) {
+          if constexpr (ES == 4) {
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+              if (mk[w]) corr += (double)(rf - __uint_as_float(x[w]));
+          } else {
+            uint32_t old = 0u;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) old = __dp4a(x[w] & mk[w], 0x01010101u, old);
+            corr = (double)((int)re * __popc(m) - (int)old);
+          }
+          if (wrow)
+            wrow[(int64_t)t * rowlen + k] =
+                make_uint4((x[0] & ~mk[0]) | (rw & mk[0]), (x[1] & ~mk[1]) | (rw & mk[1]),
+                           (x[2] & ~mk[2]) | (rw & mk[2]), (x[3] & ~mk[3]) | (rw & mk[3]));
+        }
+        if constexpr (ES == 4) {
+          for (int o = L >> 1; o > 0; o >>= 1) corr += __shfl_xor_sync(0xffffffffu, corr, o);
+        } else {                               // whole numbers: 32-bit sums
+          int ci = (int)corr;
+          for (int o = L >> 1; o > 0; o >>= 1) ci += __shfl_xor_sync(0xffffffffu, ci, o);
+          corr = (double)ci;
+        }
+        if (sub == 0 && t < t_end) corr_sh[t - t_begin] += corr;
+      }
+    }
+  }
+  __syncthreads();
+  // the channel-mean series of the chunk's rows
+  for (int t = t_begin + tid; t < t_end; t += flag::kApplyThreads) {
+    double rsum;
+    if (a.nslab == 1) {
+      rsum = a.ts[(int64_t)b * T + t];
+    } else {
+      rsum = 0.0;
+#pragma unroll 8
+      for (int s = 0; s < a.nslab; ++s) rsum += a.rowsum[((int64_t)b * a.nslab + s) * T + t];
+    }
+    a.ts[(int64_t)b * T + t] = (float)((rsum + corr_sh[t - t_begin]) / C);
   }
   // the beam's last CTA makes the time-series decisions
   __threadfence();
@@ -725,19 +1051,33 @@ __global__ void __launch_bounds__(flag::kApplyThreads) flag_apply_kernel(FlagArg
       grp_radix_select(tmp, a.ts_base, kmed, hist, sel, tid, flag::kApplyThreads, 1);
   const float lim = a.ts_thresh * mad;
   int nts = 0;
-  for (int t = tid; t < T; t += flag::kApplyThreads) {
-    const uint8_t f = (tb[t] - med) > lim ? 1 : 0;
-    mb[t] = f;
-    nts += f;
+  // 32 rows per warp and step, eight steps of loads in flight; a warp sets its
+  // own flagged rows from its lanes' votes (read back from memory row by row
+  // they took most of this kernel: 500 of 700 us for 16,384 rows)
+  for (int t0 = 32 * warp; t0 < T; t0 += 8 * 32 * nw) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int t = t0 + u * 32 * nw + lane;
+      v[u] = t < T ? __ldcg(tb + t) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int t = t0 + u * 32 * nw + lane;
+      const bool f = t < T && (v[u] - med) > lim;
+      if (t < T) mb[t] = f ? 1 : 0;
+      uint32_t votes = __ballot_sync(0xffffffffu, f);
+      if (lane == 0) nts += __popc(votes);
+      if (!xw) continue;
+      while (votes) {
+        const int i = __ffs(votes) - 1;
+        votes &= votes - 1u;
+        E *row = xw + ((int64_t)b * T + (t - lane + i)) * C;
+        for (int c = G + lane; c < C - G; c += 32) row[c] = re;
+      }
+    }
   }
   if (nts && a.counts) atomicAdd(a.counts + 1, nts);
-  if (!xw) return;
-  __syncthreads();   // the row flags written above are read back by other threads
-  for (int t = warp; t < T; t += nw) {
-    if (!mb[t]) continue;
-    E *row = xw + ((int64_t)b * T + t) * C;
-    for (int c = G + lane; c < C - G; c += 32) row[c] = re;
-  }
 }
 
 // fix_zspec (:114-170) over naver blocks of history: per (beam, channel),
@@ -787,52 +1127,66 @@ __global__ void flag_medcalc_kernel(float *arr0, float *arr1, int nbeam, int nch
 }
 
 // ---------------------------------------------------------------- launchers
-static int stage_rows(const FlagArgs &a, int es) {
-  const int cs = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
-  int lim = flag::kStageTarget / (cs * es);
-  if (lim > flag::kStatThreads) lim = flag::kStatThreads;
-  if (lim > a.tbin) lim = a.tbin;
-  for (int d = lim; d >= 1; --d)
-    if (a.tbin % d == 0 && (!a.pix_sum || d % a.tds == 0)) return d;
-  return 0;
-}
-
 bool flag_shape_ok(const FlagArgs &a) {
   const bool u8 = a.xu8 != nullptr;
   const int es = u8 ? 1 : 4;
   const void *x = u8 ? (const void *)a.xu8 : (const void *)a.x;
   if (!x || a.nchan < 4 || a.nchan > flag::kMaxChan || a.tbin < 1 || a.ntime < 1) return false;
   if ((a.nchan * es) % 16 || (reinterpret_cast<uintptr_t>(x) & 15u)) return false;
+  // (pixel rows of at most 256 samples and 24 KB)
   if (a.pix_sum && (u8 || a.nchan > kFlagSlab || a.tds < 1 || a.tbin % a.tds ||
-                    a.ntime % a.tbin))
+                    a.ntime % a.tbin || a.tds > 256 || (size_t)a.tds * a.nchan * 4 > 24576))
     return false;
-  // uint8 sums are 32-bit: at most 32768 rows per thread (P of the full slab)
+  // uint8 sums are 32-bit: a lane's share of the rows, as before at most
+  // 32768 of an eighth (more in the narrowest slabs, whose passes hold more rows)
   const int cs = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
   const int P = flag::kStatThreads / (cs / 4);
   if (u8 && (a.ntime + P - 1) / P > 32768) return false;
-  FlagArgs t = a;
-  return stage_rows(t, es) > 0;
+  return true;
 }
 
-// The largest layout over the launch's slabs: the full slab width cs and,
-// when nchan is not a multiple of it, the narrower last slab (whose P x cs
-// bin partials can exceed the full slab's).  Kept tight: at 48 channels two
-// CTAs must share an SM.
+// The largest layout over the launch's slabs: the full slab width and, when
+// nchan is not a multiple of it, the narrower last slab.
 static size_t stats_smem(const FlagArgs &a, int es) {
-  const int cs = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
-  const int last = a.nchan > kFlagSlab ? a.nchan % kFlagSlab : 0;
-  auto bp = [](int w) { return (size_t)(flag::kStatThreads / (w / 4)) * w; };
-  size_t nbp = bp(cs);
-  if (last && bp(last) > nbp) nbp = bp(last);
-  const size_t stage = ((size_t)a.rs * cs * es + 127) & ~(size_t)127;
-  // row partials (int for uint8, double for FP32), bin partials, scaley
-  // constants, and for scaled uint8 the [256][cs] table
-  const size_t rsb = ((size_t)(es == 1 ? 4 : 8) * a.rs * ((cs / 4) | 1) + 15) & ~(size_t)15;
-  const size_t stats = flag::kStages * stage + rsb + sizeof(double) * (nbp + cs) +
-                       sizeof(float) * 2 * cs + (es == 1 && a.spec0 ? (size_t)256 * cs : 0);
+  const int batch = es == 1 ? flag::batch<uint8_t>() : flag::batch<float>();
+  const int bx = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
+  const int rpw = 32 / (bx / 4);
+  const size_t stage = ((size_t)batch * rpw * bx * es + 127) & ~(size_t)127;
+  auto layout = [&](int cs) {
+    const size_t acc = es == 1 ? 4 : 8;
+    return flag::kWarps * (a.ring * stage + flag_rowbuf(cs, batch, rpw, (int)acc)) +
+           acc * 2 * flag::kWarps * cs + sizeof(double) * cs + sizeof(float) * 2 * cs +
+           (es == 1 && a.spec0 ? (size_t)256 * cs : 0);
+  };
+  size_t n = layout(bx);
+  if (a.nchan > kFlagSlab && a.nchan % kFlagSlab) {
+    const size_t l = layout(a.nchan % kFlagSlab);
+    if (l > n) n = l;
+  }
   // the channel decisions reuse the buffer: 12 nchan floats + nchan bytes
   const size_t dec = a.decide ? sizeof(float) * 12 * (size_t)a.nchan + a.nchan : 0;
-  return stats > dec ? stats : dec;
+  return n > dec ? n : dec;
+}
+
+// Time chunks per (slab, beam): enough CTAs to fill the GPU where there are
+// few beams, none where a chunk would have fewer than eight bins (a warp then
+// has part of a bin), or 1,024 rows of scaled uint8 (its table is 3 us of
+// work).
+int flag_chunks(int nbeam, int ntime, int nchan, int tbin, bool table) {
+  const int64_t ctas = (int64_t)nbeam * ((nchan + kFlagSlab - 1) / kFlagSlab);
+  const int nbins = ntime / tbin;
+  int64_t n = flag::kTargetCtas / ctas;   // (one wave of CTAs)
+  if (n > nbins / 8) n = nbins / 8;
+  if (table && n > ntime / 1024) n = ntime / 1024;
+  if (n > kFlagMaxChunks) n = kFlagMaxChunks;
+  return n < 1 ? 1 : (int)n;
+}
+
+size_t flag_part_bytes(int nbeam, int ntime, int nchan, int tbin, bool table) {
+  const int n = flag_chunks(nbeam, ntime, nchan, tbin, table);
+  return n > 1 ? sizeof(double) * (size_t)nbeam * ((nchan + kFlagSlab - 1) / kFlagSlab) * n *
+                     flag::kPartFields * kFlagSlab
+               : 0;
 }
 
 // The library-wide error word of flagger launches made without a context
@@ -853,8 +1207,8 @@ static int *flag_err_word() {
 }
 
 // The filterbank as a 2-D tensor [nbeam * ntime rows][nchan] of its element
-// type, boxes [rs rows][min(nchan, 128) channels], zero fill past nchan.
-static int encode_filterbank_map(CUtensorMap *map, const FlagArgs &a) {
+// type, boxes [brows rows][min(nchan, 128) channels], zero fill past nchan.
+static int encode_filterbank_map(CUtensorMap *map, const FlagArgs &a, int brows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (!fn) return -1;
   const bool u8 = a.xu8 != nullptr;
@@ -862,7 +1216,7 @@ static int encode_filterbank_map(CUtensorMap *map, const FlagArgs &a) {
   const int bx = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
   const cuuint64_t dims[2] = {(cuuint64_t)a.nchan, (cuuint64_t)a.nbeam * (cuuint64_t)a.ntime};
   const cuuint64_t strides[1] = {(cuuint64_t)a.nchan * es};
-  const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)a.rs};
+  const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)brows};
   const cuuint32_t estr[2] = {1u, 1u};
   void *base = u8 ? (void *)a.xu8 : (void *)a.x;
   const CUresult r = fn(map, u8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
@@ -876,26 +1230,39 @@ int launch_flag_stats(FlagArgs a, cudaStream_t st) {
   if (!flag_shape_ok(a)) return -1;
   const bool u8 = a.xu8 != nullptr;
   const int es = u8 ? 1 : 4;
-  a.rs = stage_rows(a, es);
   a.nslab = (a.nchan + kFlagSlab - 1) / kFlagSlab;
   if (a.nslab > 1 && !a.rowsum) return -1;
+  a.nchunk = a.part && a.ctr ? flag_chunks(a.nbeam, a.ntime, a.nchan, a.tbin, u8 && a.spec0) : 1;
+  if (a.nchunk > 1 && !a.decide &&
+      cudaMemsetAsync(a.ctr, 0, sizeof(int) * flag_ctr_ints(a.nbeam, a.nchan), st) != cudaSuccess)
+    return -2;
   if (!a.err) a.err = flag_err_word();
   if (!a.err) return -2;
   if (!a.wait_limit_ns) a.wait_limit_ns = 1000000000ull;
+  const int bx = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
+  const int brows = (u8 ? flag::batch<uint8_t>() : flag::batch<float>()) * (32 / (bx / 4));
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
-  if (encode_filterbank_map(&map, a) != 0) return -2;
-  const size_t sh = stats_smem(a, es);
-  const dim3 grid(a.nslab, a.nbeam);
-  if (u8) {
-    static SmemAttrOnce attr;
-    if (smem_attr_once(attr, flag_stats_kernel<uint8_t>, 160 * 1024) != cudaSuccess) return -2;
-    flag_stats_kernel<uint8_t><<<grid, flag::kStatThreads, sh, st>>>(map, a);
-  } else {
-    static SmemAttrOnce attr;
-    if (smem_attr_once(attr, flag_stats_kernel<float>, 160 * 1024) != cudaSuccess) return -2;
-    flag_stats_kernel<float><<<grid, flag::kStatThreads, sh, st>>>(map, a);
-  }
+  if (encode_filterbank_map(&map, a, brows) != 0) return -2;
+  // as deep a ring as lets two CTAs share an SM
+  size_t sh = 0;
+  for (a.ring = flag::kMaxRing; a.ring >= 2; --a.ring)
+    if ((sh = stats_smem(a, es)) <= 112 * 1024 || a.ring == 2) break;
+  const dim3 grid(a.nslab * a.nchunk, a.nbeam);
+  // full slabs, or the one slab of a 48-channel subband, have their own forms
+  const int kind = a.nchan % kFlagSlab == 0 ? 2 : a.nchan == 48 ? 1 : 0;
+  void (*const kernels[3][3])(const CUtensorMap, FlagArgs) = {
+      {flag_stats_kernel<uint8_t, false, 0>, flag_stats_kernel<uint8_t, false, 12>,
+       flag_stats_kernel<uint8_t, false, 32>},
+      {flag_stats_kernel<float, true, 0>, flag_stats_kernel<float, true, 12>,
+       flag_stats_kernel<float, true, 32>},
+      {flag_stats_kernel<float, false, 0>, flag_stats_kernel<float, false, 12>,
+       flag_stats_kernel<float, false, 32>}};
+  const int row = u8 ? 0 : a.pix_sum ? 1 : 2;
+  auto kernel = kernels[row][kind];
+  static SmemAttrOnce attr[9];
+  if (smem_attr_once(attr[3 * row + kind], kernel, 160 * 1024) != cudaSuccess) return -2;
+  kernel<<<grid, flag::kStatThreads, sh, st>>>(map, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -911,7 +1278,9 @@ int launch_flag(const FlagArgs &a0, cudaStream_t st) {
   a.ts_mean = 0;
   a.decide = 1;
   a.nslab = (a.nchan + kFlagSlab - 1) / kFlagSlab;
-  if (cudaMemsetAsync(a.ctr, 0, sizeof(int) * flag_ctr_ints(a.nbeam), st) != cudaSuccess) return -2;
+  if (cudaMemsetAsync(a.ctr, 0, sizeof(int) * (a.part ? flag_ctr_ints(a.nbeam, a.nchan)
+                                                    : flag_ctr_chunk(a.nbeam)), st) != cudaSuccess)
+    return -2;
   int rc = launch_flag_stats(a, st);
   if (rc != 0) return rc;
   const bool u8 = a.xu8 != nullptr;
@@ -1238,7 +1607,7 @@ extern "C" int dsax_flag_noalloc(const dsax_flag_params *p, const float *x, cons
     return DSAX_ERR_ARG;
   const long long nbc = (long long)B * C, nbt = (long long)B * T;
   // spec, var, max, pp, ts, the two flag counts, the launches' completion counters
-  const long long need = 4 * nbc + nbt + 2 + (long long)flag_ctr_ints(B);
+  const long long need = 4 * nbc + nbt + 2 + 2 * (long long)B + 2;
   if (need > kNoAllocScratchFloats) return DSAX_ERR_ARG;   // beyond the fixed 6 MiB
   if (C % 4 || (reinterpret_cast<uintptr_t>(x) & 15u)) return DSAX_ERR_ARG;
   int dev = -1;
@@ -1257,6 +1626,12 @@ extern "C" int dsax_flag_noalloc(const dsax_flag_params *p, const float *x, cons
   a.spec = s; a.var = s + nbc; a.maxs = s + 2 * nbc; a.pp = s + 3 * nbc; a.ts = s + 4 * nbc;
   a.counts = reinterpret_cast<int *>(s + 4 * nbc + nbt);
   a.ctr = a.counts + 2;
+  // time chunks where the array has room for their counters and partial results
+  const long long nctr = (long long)flag_ctr_ints(B, C);
+  const long long opart = (4 * nbc + nbt + 2 + nctr + 1) & ~1ll;
+  const size_t npart = flag_part_bytes(B, T, C, p->tbin, false);
+  if (npart && opart + (long long)(npart / 4) <= kNoAllocScratchFloats)
+    a.part = reinterpret_cast<double *>(s + opart);
   // the counters accumulate with atomics: clear them (the array keeps the
   // previous call's values)
   if (cudaMemsetAsync(a.counts, 0, 2 * sizeof(int), st) != cudaSuccess) return DSAX_ERR_CUDA;

@@ -62,6 +62,7 @@ struct dsax_flag_state {
   void *noise = nullptr;
   uint8_t *dmask = nullptr; // masks when the caller passes none (device mode)
   int *ctr = nullptr;       // completion counters of the flagger launches
+  double *part = nullptr;   // partial results of their time chunks
 };
 
 extern "C" {
@@ -112,9 +113,10 @@ int dsax_flag(dsax_ctx *c, const dsax_flag_params *p, const float *x, const floa
   const size_t nstat = 4 * nbc + nbt;
   const size_t nrow = nslabs(C) > 1 ? (size_t)B * nslabs(C) * T : 0;
   int rc;
-  const size_t nctr = flag_ctr_ints(B);
-  if ((rc = ensure_buffer(c, c->aux[AUX_FLAG_STATS], (nstat + nrow + 2 + nctr) * 4 + 64,
-                          "flag statistics")) != DSAX_OK)
+  const size_t nctr = flag_ctr_ints(B, C);
+  const size_t opart = ((nstat + nrow + 2 + nctr) * 4 + 64 + 255) / 256 * 256;
+  const size_t npart = flag_part_bytes(B, T, C, p->tbin, false);
+  if ((rc = ensure_buffer(c, c->aux[AUX_FLAG_STATS], opart + npart, "flag statistics")) != DSAX_OK)
     return rc;
   FlagArgs a{};
   fill_args(a, p);
@@ -128,6 +130,8 @@ int dsax_flag(dsax_ctx *c, const dsax_flag_params *p, const float *x, const floa
   a.rowsum = nrow ? scratch + nstat : nullptr;
   int *dcounts = reinterpret_cast<int *>(scratch + nstat + nrow);
   a.ctr = dcounts + 2;
+  if (npart)
+    a.part = reinterpret_cast<double *>(static_cast<uint8_t *>(c->aux[AUX_FLAG_STATS].ptr) + opart);
   a.counts = (mem == DSAX_MEM_DEVICE && counts) ? counts : dcounts;
   cudaError_t e = cudaMemsetAsync(a.counts, 0, 2 * sizeof(int), c->stream);
   if (e != cudaSuccess) return cuda_check(c, e, "clear counts");
@@ -188,7 +192,10 @@ int dsax_flag_state_create(dsax_ctx *c, const dsax_flag_params *p,
   const size_t off_noise = off_d + 256;
   const size_t off_mask = ((off_noise + (size_t)T * C * es + 255) / 256) * 256;
   const size_t off_ctr = ((off_mask + bc + bt + 255) / 256) * 256;
-  const size_t total = off_ctr + sizeof(int) * flag_ctr_ints(B);
+  // (the chunks' partial results: the larger of the measured and the scaled passes')
+  const size_t off_part = ((off_ctr + sizeof(int) * flag_ctr_ints(B, C) + 255) / 256) * 256;
+  const size_t npart = flag_part_bytes(B, T, C, p->tbin, false);
+  const size_t total = off_part + npart;
   cudaError_t e = cudaMalloc(&st->buf.ptr, total);
   if (e != cudaSuccess) {
     delete st;
@@ -211,6 +218,7 @@ int dsax_flag_state_create(dsax_ctx *c, const dsax_flag_params *p,
   st->noise = base + off_noise;
   st->dmask = base + off_mask;
   st->ctr = reinterpret_cast<int *>(base + off_ctr);
+  st->part = npart ? reinterpret_cast<double *>(base + off_part) : nullptr;
   // zero everything (oldspec starts at 0, as h_oldspec does at :1214), then
   // the levels at 1 (:1234) and the noise block
   if ((e = cudaMemsetAsync(st->buf.ptr, 0, total, c->stream)) != cudaSuccess) {
@@ -300,6 +308,7 @@ int dsax_flag_clean(dsax_ctx *c, dsax_flag_state *st, void *data, uint8_t *chanm
   a.counts = st->counts;
   a.status = st->status;
   a.ctr = st->ctr;
+  a.part = st->part;
   a.mn = st->cp.mn;
   a.sig = st->cp.sig;
   a.bpwr = st->bpwr;

@@ -118,7 +118,9 @@ struct FlagArgs {
   int tds = 0;
   // statistics-pass geometry, set by the launcher
   int nslab = 1;                 // channel slabs of kFlagSlab channels (CTAs per beam)
-  int rs = 0;                    // rows per pipeline stage (divides tbin)
+  int nchunk = 1;                // time chunks per (slab, beam)
+  int ring = 2;                  // boxes of a statistics warp's ring
+  double *part = nullptr;        // partial results of the chunks (flag_part_bytes), or null: one chunk
   int ts_mean = 0;               // 1: the statistics pass writes ts = row mean (no apply pass)
   // data path (src/gpu_flagger.cu:1290-1410)
   int clean = 0;                 // 1: replace flagged columns / rows in xw / xw8
@@ -133,22 +135,36 @@ struct FlagArgs {
   double *tpwr_out = nullptr;    // this block's total power
   int *status = nullptr;         // [0] = 1 when the block was replaced by noise
   const void *noise = nullptr;   // replacement block [ntime][nchan] (element type of x)
-  // completion counters, [2 nbeam + 2] ints zeroed by launch_flag: per-beam
-  // slab CTAs done, per-beam apply CTAs done, CTAs of the statistics grid
-  // done (the last arrival of each does the next step; nothing spins)
+  // completion counters (flag_ctr_ints) zeroed by launch_flag: per-beam slab
+  // CTAs done, per-beam apply CTAs done, CTAs of the statistics grid done, and
+  // per (beam, slab) chunk CTAs done (the last arrival of each does the next
+  // step; nothing spins)
   int *ctr = nullptr;
   int decide = 0;                // statistics pass also makes the channel decisions
-  // bounded waits of the statistics pass (TMA stages): where a wait that
-  // ran out is recorded (a context's error word; null: a library-wide word)
-  // and the bound (0: 1 s)
+  // bounded waits of the statistics pass (TMA boxes): where a wait that ran
+  // out is recorded (a context's error word; null: a library-wide word) and
+  // the bound (0: 1 s)
   int *err = nullptr;
   unsigned long long wait_limit_ns = 0;
 };
 
-// ints of FlagArgs::ctr for nbeam beams
-inline size_t flag_ctr_ints(int nbeam) { return 2 * (size_t)nbeam + 2; }
-
 constexpr int kFlagSlab = 128;   // channels per statistics CTA
+constexpr int kFlagMaxChunks = 64;
+
+// ints of FlagArgs::ctr, and where its chunk counters begin
+inline __host__ __device__ size_t flag_ctr_chunk(int nbeam) { return 2 * (size_t)nbeam + 2; }
+inline size_t flag_ctr_ints(int nbeam, int nchan) {
+  return flag_ctr_chunk(nbeam) + (size_t)nbeam * ((nchan + kFlagSlab - 1) / kFlagSlab);
+}
+// Bytes of FlagArgs::part for a shape (0: not chunked); table: scaled uint8.
+size_t flag_part_bytes(int nbeam, int ntime, int nchan, int tbin, bool table);
+// Bytes of a statistics warp's row buffer (batch * rpw rows of partial sums of
+// `acc` bytes, odd stride), and at least its share of the [8 rpw][cs] FP64
+// totals that reuse it; a multiple of 16.
+inline __host__ __device__ int flag_rowbuf(int cs, int batch, int rpw, int acc) {
+  const int rows = batch * rpw * ((cs / 4) | 1) * acc, tot = rpw * cs * 8;
+  return ((rows > tot ? rows : tot) + 15) & ~15;
+}
 
 int launch_flag(const FlagArgs &a, cudaStream_t st);
 // Statistics pass only (spec, var, max, pp, ts and the optional pixel sums).

@@ -78,15 +78,23 @@ struct LfScratch {
   float *stats, *pix;   // statistics pass: spec, var, max, pp [B][W]; ts [B][T]; pixel sum, max
   uint8_t *L;
   double *loss;
+  int *ctr;             // completion counters and partial results of the statistics chunks
+  double *spart;
 };
 
-int lf_scratch(dsax_ctx *c, int B, int H, int W, int T, LfScratch &s) {
+int lf_scratch(dsax_ctx *c, int B, int H, int W, int T, int tbin, LfScratch &s) {
   const size_t px = (size_t)B * H * W;
   const size_t nstat = (size_t)4 * B * W + (size_t)B * T;
   const size_t nf = px * (8 + 32 + 64 + 64 + 1 + 1 + 64 + 64) + lf_part_floats(B, H) + nstat + 2 * px;
-  int rc = ensure_buffer(c, c->aux[AUX_LF_SCRATCH], nf * 4 + px + 64 + 64, "learned-flagger scratch");
+  auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+  const size_t octr = up(nf * 4 + px + 64 + 64);
+  const size_t ospart = up(octr + sizeof(int) * flag_ctr_ints(B, W));
+  int rc = ensure_buffer(c, c->aux[AUX_LF_SCRATCH], ospart + flag_part_bytes(B, T, W, tbin, false),
+                         "learned-flagger scratch");
   if (rc != DSAX_OK) return rc;
   float *f = static_cast<float *>(c->aux[AUX_LF_SCRATCH].ptr);
+  s.ctr = reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(f) + octr);
+  s.spart = reinterpret_cast<double *>(reinterpret_cast<uint8_t *>(f) + ospart);
   s.loss = reinterpret_cast<double *>(f);  f += 16;
   s.F = f;  f += px * 8;
   s.a1 = f; f += px * 32;
@@ -122,6 +130,8 @@ int lf_make_features(const dsax_flag_params *p, const float *x, int tds, const L
   a.pix_max = s.pix + (size_t)B * H * C;
   a.tds = tds;
   a.ts_mean = 1;
+  a.ctr = s.ctr;
+  a.part = s.spart;
   if (!flag_shape_ok(a)) return -1;
   int rc = launch_flag_stats(a, st);
   if (rc != 0) return rc;
@@ -179,7 +189,7 @@ int dsax_lf_features(dsax_ctx *c, const float *x, const dsax_flag_params *p, int
   if (rc != DSAX_OK) return rc;
   DeviceGuard g(c->device);
   LfScratch s;
-  if ((rc = lf_scratch(c, p->nbeam, p->ntime / tds, p->nchan, p->ntime, s)) != DSAX_OK) return rc;
+  if ((rc = lf_scratch(c, p->nbeam, p->ntime / tds, p->nchan, p->ntime, p->tbin, s)) != DSAX_OK) return rc;
   if (lf_make_features(p, x, tds, s, F, nullptr, c->stream) != 0)
     return cuda_check(c, cudaGetLastError(), "feature launch");
   return DSAX_OK;
@@ -195,7 +205,7 @@ int dsax_lf_train_step(dsax_ctx *c, const float *x, const uint8_t *chanmask, con
   DeviceGuard g(c->device);
   const int B = p->nbeam, H = p->ntime / tds, W = p->nchan;
   LfScratch s;
-  if ((rc = lf_scratch(c, B, H, W, p->ntime, s)) != DSAX_OK) return rc;
+  if ((rc = lf_scratch(c, B, H, W, p->ntime, p->tbin, s)) != DSAX_OK) return rc;
   LfNet &net = *c->lf;
   float *acts[5] = {s.F, s.a1, s.a2, s.a3, s.z};
   const int nvalid = B * H * (W - 2 * p->guard);
@@ -236,7 +246,7 @@ int dsax_flag_learned(dsax_ctx *c, const float *x, const dsax_flag_params *p, in
   DeviceGuard g(c->device);
   const int B = p->nbeam, H = p->ntime / tds, W = p->nchan;
   LfScratch s;
-  if ((rc = lf_scratch(c, B, H, W, p->ntime, s)) != DSAX_OK) return rc;
+  if ((rc = lf_scratch(c, B, H, W, p->ntime, p->tbin, s)) != DSAX_OK) return rc;
   LfNet &net = *c->lf;
   const float *xd = x;
   const size_t px = (size_t)B * H * W;
