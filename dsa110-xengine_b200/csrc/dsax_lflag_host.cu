@@ -35,7 +35,8 @@ int ensure_net(dsax_ctx *c) {
   const int np = lf_nparams();
   int rc = ensure_buffer(c, c->aux[AUX_LF_STATE], sizeof(float) * 4 * np, "learned-flagger state");
   if (rc != DSAX_OK) return rc;
-  rc = ensure_buffer(c, c->aux[AUX_LF_WLAYOUT], sizeof(float) * 2 * np, "learned-flagger layouts");
+  const int npa = (np + 3) & ~3;   // both layouts on 16-byte boundaries
+  rc = ensure_buffer(c, c->aux[AUX_LF_WLAYOUT], sizeof(float) * 2 * npa, "learned-flagger layouts");
   if (rc != DSAX_OK) return rc;
   float *base = static_cast<float *>(c->aux[AUX_LF_STATE].ptr);
   n.params = base;
@@ -49,7 +50,7 @@ int ensure_net(dsax_ctx *c) {
     n.gw[l] = n.grads + lf_w_offset(l);
     n.gb[l] = n.grads + lf_b_offset(l);
     n.wt[l] = lay + lf_w_offset(l);
-    n.wf[l] = lay + np + lf_w_offset(l);
+    n.wf[l] = lay + npa + lf_w_offset(l);
   }
   cudaMemsetAsync(base, 0, sizeof(float) * 4 * np, c->stream);
   n.step = 0;
