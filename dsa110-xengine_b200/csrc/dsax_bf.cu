@@ -531,6 +531,11 @@ __global__ void __launch_bounds__(bf::threads(kEpiW), 1) bf_kernel(BfArgs a) {
 //   warp  16  : TMEM allocation (both CTAs), own weight tile (both CTAs),
 //               MMA issue (even CTA); stage / accumulator / weight-drain
 //               releases are multicast commits to both CTAs
+// An epilogue warp frees the accumulator as soon as its last columns are in
+// registers, before it squares them (the MMAs two units on wait for that), and
+// a unit's outputs (up to four) are combined together, with one barrier each
+// time instead of two per output: full block BF16 372 -> 361 us, FP8 342 ->
+// 324; 200 channels, 128 beams, four packets per output 138 -> 105 (FP8).
 // Cross-CTA arrivals use the default release-at-CTA-scope form (the form
 // of the CUDA templates' CTA-pair pipelines); release at cluster scope
 // cost a memory barrier per arrival and measured about 25 % slower.
@@ -580,7 +585,8 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
   __shared__ __align__(8) uint64_t final_bar;           // both: every MMA done
   __shared__ uint32_t tmem_base_sh;
   __shared__ volatile int abort_sh;
-  __shared__ float red[kEpiW / 4][128];   // one output's row partials per column share
+  // the row partials per column share of up to four outputs, two sets in turn
+  __shared__ float red[2][4][kEpiW / 4][128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -662,8 +668,13 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
         shift_add[e] = a0 | (a0 << 8) | (a1 << 16) | (a1 << 24);
       }
     }
+    int sg = (u_lo >> 1) / npg, spg = (u_lo >> 1) - sg * npg;   // next group to stage
     auto stage_group = [&](int r) {
-      const int g = r / npg, pg = r % npg;
+      const int g = sg, pg = spg;
+      if (++spg == npg) {
+        spg = 0;
+        ++sg;
+      }
       const int p = pg * kPktPerStage + q;
       const uint32_t slot = (uint32_t)(r % kRD) * bfp::kRawBytes;
 #pragma unroll
@@ -783,6 +794,8 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
     const int pgs_per_out = a.ppo > kPktPerStage ? a.ppo / kPktPerStage : 1;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     float bpow = 0.f;
+    int g = (u_lo >> 1) / npg, pg = (u_lo >> 1) - g * npg, par = 0;
+    const int et = 32 * (warp - 8) + lane;
     for (int u = u_lo, i = 0; u < u_hi; ++u, ++i) {
       const int b = i & 1;
       const uint32_t ph = (uint32_t)(i >> 1) & 1u;
@@ -791,6 +804,14 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
       tc_fence_after();
       ok = __all_sync(0xffffffffu, ok && !abort_sh);
       const uint32_t taddr = tmem + ((uint32_t)(32 * qq) << 16) + (uint32_t)b * 256u;
+      // the accumulator goes back once its last columns are in registers: the
+      // MMAs two units on wait for it
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);
+      };
+      if (!ok) release();
 #pragma unroll
       // kLdG 32-column TMEM loads in flight per wait
       for (int cc = 0; cc < (ok ? kCW : 0); cc += kLdG) {
@@ -798,6 +819,7 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
 #pragma unroll
         for (int gi = 0; gi < kLdG; ++gi) tmem_ld32(taddr + 32u * (half * kCW + cc + gi), r0[gi]);
         tmem_wait_ld();
+        if (cc + kLdG >= kCW) release();
 #pragma unroll
         for (int gi = 0; gi < kLdG; ++gi) {
           const int c = half * kCW + cc + gi;
@@ -831,53 +853,58 @@ __global__ void __launch_bounds__(bfp::threads(kEpiW), 1) bf_pair_kernel(BfArgs 
           else acc[3] += sq;
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty0 + 8u * (uint32_t)b);
 
-      int g, pg, pol;
-      bf_decode(u, npg, g, pg, pol);
+      const int pol = u & 1;
       if (pol == 1 && ((pg + 1) % pgs_per_out) == 0) {
         // rows m and m + 64 hold Re and Im of the same beam; the column
-        // shares of a row are summed through shared memory, one output at
-        // a time
-        const int beam = 64 * bt + m;
+        // shares of a row are summed through shared memory, all of the unit's
+        // outputs at once.  One barrier: the set written here is written again
+        // after the next output's barrier, which nobody passes before every
+        // warp has read this one.
 #pragma unroll
-        for (int sI = 0; sI < 4; ++sI) {
-          if (sI >= nsub) break;
-          red[half][m] = acc[sI];
-          named_bar(1, kEpiThreads);
-          if (half == 0 && m < 64 && !abort_sh) {
-            float Ps = red[0][m] + red[0][m + 64];
+        for (int sI = 0; sI < 4; ++sI)
+          if (sI < nsub) red[par][sI][half][m] = acc[sI];
+        named_bar(1, kEpiThreads);
+        for (int id = abort_sh ? 64 * nsub : et; id < 64 * nsub; id += kEpiThreads) {
+          const int sI = id >> 6, mm = id & 63, beam = 64 * bt + mm;
+          float Ps = red[par][sI][0][mm] + red[par][sI][0][mm + 64];
 #pragma unroll
-            for (int h2 = 1; h2 < kEpiW / 4; ++h2) Ps += red[h2][m] + red[h2][m + 64];
-            const float P = Ps * a.pscale;
-            const int to = a.ppo <= kPktPerStage ? pg * nsub + sI : pg / pgs_per_out;
-            const int64_t o = ((int64_t)to * a.nbeam + beam) * ngrp + g;
-            if (a.out_f32) a.out_f32[o] = P;
-            if (a.out_fb) a.out_fb[((int64_t)beam * (a.npkt / a.ppo) + to) * ngrp + g] = P;
-            if (a.out_u8) {
-              int v = a.agc_scale ? __float2int_rn(P * __ldg(a.agc_scale + beam)) / 2
-                                  : __float2int_rn(P * a.scale);
-              a.out_u8[o] = (uint8_t)(v < 0 ? 0 : (v > 255 ? 255 : v));
-            }
-            bpow += P;
+          for (int h2 = 1; h2 < kEpiW / 4; ++h2) Ps += red[par][sI][h2][mm] + red[par][sI][h2][mm + 64];
+          const float P = Ps * a.pscale;
+          const int to = a.ppo <= kPktPerStage ? pg * nsub + sI : pg / pgs_per_out;
+          const int64_t o = ((int64_t)to * a.nbeam + beam) * ngrp + g;
+          if (a.out_f32) a.out_f32[o] = P;
+          if (a.out_fb) a.out_fb[((int64_t)beam * (a.npkt / a.ppo) + to) * ngrp + g] = P;
+          if (a.out_u8) {
+            int v = a.agc_scale ? __float2int_rn(P * __ldg(a.agc_scale + beam)) / 2
+                                : __float2int_rn(P * a.scale);
+            a.out_u8[o] = (uint8_t)(v < 0 ? 0 : (v > 255 ? 255 : v));
           }
-          named_bar(1, kEpiThreads);
+          bpow += P;
         }
+        par ^= 1;
         acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
       }
+      if (pol == 1 && ++pg == npg) {
+        pg = 0;
+        ++g;
+      }
     }
-    if (a.beam_power && half == 0 && m < 64 && bpow != 0.f)
-      atomicAdd(a.beam_power + 64 * bt + m, bpow);
+    // (a thread's outputs are all of beam et % 64: kEpiThreads is a multiple of 64)
+    if (a.beam_power && bpow != 0.f) atomicAdd(a.beam_power + 64 * bt + (et & 63), bpow);
   } else {
     // ------------------------------------------------------------ weights + MMA
     if (lane == 0) {
       int cur_g = -1;
       uint32_t nload = 0, ndrain = 0;
+      const int g_lo = (u_lo >> 1) / npg;
+      int g = g_lo, u_g = 2 * npg * (g_lo + 1);   // the channel group and its end
       for (int u = u_lo, i = 0; u < u_hi && !abort_sh; ++u, ++i) {
-        int g, pg, pol;
-        bf_decode(u, npg, g, pg, pol);
+        if (u == u_g) {
+          ++g;
+          u_g += 2 * npg;
+        }
+        const int pol = u & 1;
         if (g != cur_g) {
           if (i > 0) {  // no MMA may still read either CTA's old weights
             if (leader) umma_commit_pair(&wdrain_bar, bfp::kBoth);

@@ -453,58 +453,61 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
     for (int k = 1; k < rpw; ++k) t += __shfl_sync(0xffffffffu, bs[j], (lane + k * G4) & 31);
     return t;
   };
-  if (bin1 - bin0 >= kWarps) {
-    run((bin0 + warp) * TB, TB, kWarps * TB, (bin1 - bin0 - warp + kWarps - 1) / kWarps, [&]() {
+  // Segments: all of the warp's whole bins in one, or, with fewer bins than
+  // warps, one per bin (an eighth of its rows, in passes or pixel rows, per
+  // warp; the bin's sums combined by the CTA); then the rows beyond the last
+  // whole bin: everything but the bins.  (One loop, so that the row code exists
+  // once.)
+  const bool by_warp = bin1 - bin0 >= kWarps;
+  const int nbseg = by_warp ? 1 : bin1 - bin0;
+  const int nseg = nbseg + (chunk == a.nchunk - 1 && nbins * TB < T ? 1 : 0);
+#pragma unroll 1
+  for (int seg = 0; seg < nseg; ++seg) {
+    const bool tail = seg == nbseg, whole = by_warp && !tail;
+    int t0 = (bin0 + warp) * TB, n = TB, count = (bin1 - bin0 - warp + kWarps - 1) / kWarps;
+    if (!whole) {
+      const int s0 = tail ? nbins * TB : (bin0 + seg) * TB, len = tail ? T - s0 : TB;
+      const int unit = kPix ? a.tds : rpw;
+      const int per = ((len + unit - 1) / unit + kWarps - 1) / kWarps * unit;
+      const int r0 = min(len, warp * per), r1 = min(len, (warp + 1) * per);
+      t0 = s0 + r0;
+      n = r1 - r0;
+      count = 1;
+    }
+    run(t0, n, kWarps * TB, count, [&]() {
+      if (whole) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const Acc t = bin_total(j);
-        if (lead) {
-          Acc *e = sm_bx + 2 * warp * cs + 4 * g + j;
-          e[0] = max(e[0], t);
-          e[cs] = min(e[cs], t);
+        for (int j = 0; j < 4; ++j) {
+          const Acc t = bin_total(j);
+          if (lead) {
+            Acc *e = sm_bx + 2 * warp * cs + 4 * g + j;
+            e[0] = max(e[0], t);
+            e[cs] = min(e[cs], t);
+          }
+          s[j] += bs[j];
+          bs[j] = 0;
         }
-        s[j] += bs[j];
-        bs[j] = 0;
       }
     });
-  } else {
-    // few bins: an eighth of the rows (in passes, or pixel rows) of each per
-    // warp, the bin's sums combined by the CTA
-    const int unit = kPix ? a.tds : rpw;
-    const int units = (TB + unit - 1) / unit, per = (units + kWarps - 1) / kWarps;
-#pragma unroll 1
-    for (int bin = bin0; bin < bin1; ++bin) {
-      const int r0 = min(TB, warp * per * unit), r1 = min(TB, (warp + 1) * per * unit);
-      run(bin * TB + r0, r1 - r0, 0, 1, []() {});
-      __syncthreads();   // the row buffers become [8][cs] partial bin sums
-      Acc *const bp = reinterpret_cast<Acc *>(fs_x);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const Acc t = bin_total(j);
-        if (lead) bp[warp * cs + 4 * g + j] = t;
-        s[j] += bs[j];
-        bs[j] = 0;
-      }
-      __syncthreads();
-      for (int c = tid; c < cs; c += flag::kStatThreads) {
-        Acc t = 0;
-        for (int w = 0; w < kWarps; ++w) t += bp[w * cs + c];
-        sm_bx[c] = max(sm_bx[c], t);
-        sm_bx[cs + c] = min(sm_bx[cs + c], t);
-      }
-      __syncthreads();
-    }
-  }
-  // rows beyond the last whole bin: everything but the bins
-  if (chunk == a.nchunk - 1 && nbins * TB < T) {
-    const int n = T - nbins * TB, per = ((n + rpw - 1) / rpw + kWarps - 1) / kWarps * rpw;
-    const int r0 = min(n, warp * per), r1 = min(n, (warp + 1) * per);
-    run(nbins * TB + r0, r1 - r0, 0, 1, []() {});
+    if (whole) continue;
+    Acc *const bp = reinterpret_cast<Acc *>(fs_x);
+    if (!tail) __syncthreads();   // the row buffers become [8][cs] partial bin sums
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+      const Acc t = bin_total(j);
+      if (lead && !tail) bp[warp * cs + 4 * g + j] = t;
       s[j] += bs[j];
       bs[j] = 0;
     }
+    if (tail) continue;
+    __syncthreads();
+    for (int c = tid; c < cs; c += flag::kStatThreads) {
+      Acc t = 0;
+      for (int w = 0; w < kWarps; ++w) t += bp[w * cs + c];
+      sm_bx[c] = max(sm_bx[c], t);
+      sm_bx[cs + c] = min(sm_bx[cs + c], t);
+    }
+    __syncthreads();
   }
   __syncthreads();
   if (sabort) return;   // recorded in a.err; no statistics from this CTA
@@ -632,8 +635,8 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
 // Up to kRankMax values the element of rank k is found by counting instead (one
 // barrier for 16: of the 48 channels' decisions the four-pass select was half).
 constexpr int kRankMax = 128;
-__device__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist, uint32_t *sel,
-                                  int gtid, int gsize, int bid) {
+__device__ __forceinline__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist,
+                                                  uint32_t *sel, int gtid, int gsize, int bid) {
   if (n <= kRankMax) {
     for (int i = gtid; i < n; i += gsize) {
       const uint32_t x = ordered_key(v[i]);
@@ -694,6 +697,13 @@ __device__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist, 
   return __uint_as_float(u);
 }
 
+// The same as a call, for the channel decisions: a CTA runs them once, and what
+// they cost is mostly fetching their instructions.
+__device__ __noinline__ float grp_select_call(const float *v, int n, int k, uint32_t *hist,
+                                              uint32_t *sel, int gtid, int gsize, int bid) {
+  return grp_radix_select(v, n, k, hist, sel, gtid, gsize, bid);
+}
+
 // One window of channflag's detrend: v - lower median of x[0..kF), the median
 // by rank counting with ties by index, in registers (a thread per window;
 // with a thread per window element and shared loads it was 70 us of the 1,024
@@ -726,7 +736,7 @@ __device__ __forceinline__ void window_median(const float *x, float v, float *ou
 __device__ void grp_detrend3(float *sb0, const FlagArgs &a, int gtid, int gsize) {
   const int C = a.nchan, G = a.guard, F = a.filt, n = C - 2 * G;
   const int kf = (F + 1) / 2 - 1;
-  if (F == 21) {   // nFiltSize
+  if (F == 21 && n > kRankMax) {   // nFiltSize; few channels: not worth the unrolled code
     for (int id = gtid; id < 3 * n; id += gsize) {
       const int k = id / n, jj = id - k * n;
       float *sb = sb0 + 3 * C * k;
@@ -760,10 +770,10 @@ __device__ void grp_channflag(float thr, const FlagArgs &a, uint8_t *mask, const
                               int bid) {
   const int C = a.nchan, G = a.guard, n = C - 2 * G;
   const int k = (n + 1) / 2 - 1;
-  const float med = grp_radix_select(corr, n, k, hist, sel, gtid, gsize, bid);
+  const float med = grp_select_call(corr, n, k, hist, sel, gtid, gsize, bid);
   for (int i = gtid; i < n; i += gsize) tmp[i] = fabsf(corr[i] - med);
   named_bar(bid, gsize);
-  const float mad = grp_radix_select(tmp, n, k, hist, sel, gtid, gsize, bid);
+  const float mad = grp_select_call(tmp, n, k, hist, sel, gtid, gsize, bid);
   for (int i = gtid; i < n; i += gsize) {
     const float v = corr[i];
     if (v > thr * mad || v < -thr * mad) mask[G + i] = 1;
@@ -801,10 +811,10 @@ __device__ void flag_decide_beam(const FlagArgs &a, int b, uint8_t *smem) {
     for (int i = gtid; i < n; i += gsize) corr[i] = sb[G + i];
     named_bar(bid, gsize);
     const int k = (n + 1) / 2 - 1;
-    const float med = grp_radix_select(corr, n, k, hist[g], sel[g], gtid, gsize, bid);
+    const float med = grp_select_call(corr, n, k, hist[g], sel[g], gtid, gsize, bid);
     for (int i = gtid; i < n; i += gsize) tm[i] = fabsf(corr[i] - med);
     named_bar(bid, gsize);
-    const float mad = grp_radix_select(tm, n, k, hist[g], sel[g], gtid, gsize, bid);
+    const float mad = grp_select_call(tm, n, k, hist[g], sel[g], gtid, gsize, bid);
     const float mythr = (float)((double)a.thresh / sqrt((double)a.fbin));
     for (int j = G + gtid; j < C - G - a.fbin; j += gsize) {
       float vv = 0.0f;
