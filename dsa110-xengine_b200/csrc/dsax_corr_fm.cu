@@ -14,30 +14,34 @@
 // (N = 128, added to the first 128 columns) give Re and E = R I^T, all times
 // 256.
 //
-// Roles: unpack warps 0-7 in two groups of four that take alternate stages
+// Roles: unpack warps 0-3 in two groups of two that take alternate stages
 // (a stage is a chain of waits, loads, stores, fence and arrival of about
 // 1,000 cycles against 768 of its MMAs, so two are in flight); epilogue warps
-// 8-11, one per TMEM lane quarter; warp 12 issues the MMAs; warp 13 the TMA
+// 4-11, two per TMEM lane quarter; warp 12 issues the MMAs; warp 13 the TMA
 // boxes.
 //
 // What bounds it: shared memory.  A stage moves 1,152 128-byte wavefronts
 // (640 of operand reads, 256 of operand stores, 256 of the raw stage in and
 // out) against 768 cycles of MMAs: 56 us for the full block's 96 stages of a
-// CTA, measured 58 without the epilogue and 64 with it; 47 without the MMAs
-// and 41 for the boxes alone.  (One CTA per channel with the epilogue between
-// channels: 76.)  Stages of 64 packets 77 us, of 256 73 (half the ring); one
-// group of eight warps 66, four groups of two 64; loads straight into
-// registers instead of boxes 66.  The loops that one thread runs per stage
-// (boxes, MMAs) keep ring positions as counters: with a division by the
-// number of stages and modulo indices they took 0.3 us per stage.
+// CTA; measured 62.  (One CTA per channel with the epilogue between channels:
+// 76.)  Stages of 64 packets 77 us, of 256 73 (half the ring); loads straight
+// into registers instead of boxes 66.  The loops that one thread runs per
+// stage (boxes, MMAs) keep ring positions as counters: with a division by the
+// number of stages and modulo indices they took 0.3 us per stage.  Short
+// blocks are bound by the epilogue, a chain of loads, shuffles and stores:
+// four warps 39.8 us for 128 packets x 384 channels with the corner turn,
+// eight 28.8 (with eight unpack warps beside them registers spill: 30.9).
 //
-// Epilogue: the warp of quarter q holds rows j = 16q..16q+15 (x 2 pols) and
-// writes the outputs (i, j) for its columns i >= j as conjugates, so that the
+// Epilogue: the warps of quarter q hold rows j = 16q..16q+15 (x 2 pols) and
+// write the outputs (i, j) for their columns i >= j as conjugates, so that the
 // lanes of a store cover consecutive j: 512 contiguous bytes per store instead
 // of 16 separate 32-byte pieces.  The block i >= 48, j < 16 goes to quarter 3
-// in row order, which leaves no warp more than three 16 x 16 blocks.  Im needs
-// E and its transpose: the 32 x 32 blocks of E that are read transposed go
-// through shared memory, six and then four (24 KB).
+// in row order, which leaves no quarter more than three 16 x 16 blocks, split
+// between its two warps.  Im needs E and its transpose: the 32 x 32 blocks of E
+// that are read transposed go through shared memory, six and then four (24 KB).
+// When accumulating, a block's old values are on their way while the one before
+// it is written (loaded where they are added: 253 us against 137 for the full
+// block with the corner turn).
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -53,13 +57,13 @@ constexpr int kPkt = 128;                        // packets per stage
 constexpr uint32_t kTile = kPkt * 128;           // one operand tile (R or I)
 constexpr uint32_t kOpBytes = 2 * kTile;
 constexpr uint32_t kRawBytes = kPkt * 128;
-constexpr int kGroups = 2, kGroupWarps = 4;      // unpack warps: groups x warps of a group
+constexpr int kGroups = 2, kGroupWarps = 2;      // unpack warps: groups x warps of a group
 constexpr int kOpStages = 4, kRawStages = 4;
 // a ring slot is always the same group's: a group that skipped a phase of its
 // barrier could not tell the next one from it
 static_assert(kGroups <= kOpStages && kGroups <= kRawStages && kOpStages % kGroups == 0 && kRawStages % kGroups == 0, "ring slots of one group");
 constexpr int kUnpackWarps = kGroups * kGroupWarps;
-constexpr int kEpiWarps = 4;
+constexpr int kEpiWarps = 8;                     // two per TMEM lane quarter
 constexpr int kUnits = kPkt * 8 / (32 * kGroupWarps);   // 16-byte chunks per thread and stage
 constexpr uint32_t kScratch = 6 * 32 * 32 * 4;   // six 32 x 32 blocks of E
 constexpr int kWarpMma = kUnpackWarps + kEpiWarps, kWarpTma = kWarpMma + 1;
@@ -84,6 +88,12 @@ struct Ring {
   }
 };
 
+__device__ __forceinline__ float4 add4(float4 x, float4 y) {
+  return make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+}
+
+// kAcc: adds to vis instead of overwriting it.
+template <bool kAcc>
 __global__ void __launch_bounds__(corrfm::kThreads, 1)
     corr_fm_kernel(const __grid_constant__ CUtensorMap tmap, CorrArgs a) {
   using namespace corrfm;
@@ -171,27 +181,33 @@ __global__ void __launch_bounds__(corrfm::kThreads, 1)
     }
   } else if (warp < kWarpMma) {
     // ------------------------------------------------------------ epilogue
-    const int q = warp & 3;                          // TMEM lane quarter
+    const int q = warp & 3, hh = (warp - kUnpackWarps) >> 2;   // TMEM lane quarter, share
     uint32_t *E = reinterpret_cast<uint32_t *>(gbase + kOpStages * kOpBytes + kRawStages * kRawBytes);
     const int j = 16 * q + (lane >> 1), pj = lane & 1;
 #pragma unroll 1
     for (int fi = 0; fi < nf; ++fi) {
       const int b = fi & 1;
+      const int64_t f = (int64_t)blockIdx.x + (int64_t)fi * gridDim.x;
+      float4 *const out = reinterpret_cast<float4 *>(a.vis + f * (2080 * 8));   // 16-byte units
+      // accumulating: the old values of the warp's share of block (I, q), each
+      // set on its way while the one before is written (or waited for)
+      using Old = float4[kAcc ? 8 : 1];
+      Old oa, ob;
+      auto load_old = [&](int I, Old &o) {
+        if constexpr (kAcc) {
+#pragma unroll
+          for (int ii = 0; ii < 8; ++ii) {
+            const int i = 16 * I + 8 * hh + ii;
+            if (j <= i) o[ii] = out[i * (i + 1) + 2 * j + pj];
+          }
+        }
+      };
+      load_old(q, oa);
       bool ok = mbar_wait_bounded(&acc_full[b], (uint32_t)(fi >> 1) & 1u, &abort_sh, a.err,
                                   DEV_ERR_WAIT_ACCUM, a.wait_limit_ns);
       tc_fence_after();
       ok = __all_sync(0xffffffffu, ok && !abort_sh);
       const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)b * 256u;
-      const int64_t f = (int64_t)blockIdx.x + (int64_t)fi * gridDim.x;
-      float *vis = a.vis + f * (2080 * 8);
-      auto put = [&](int64_t o16, float4 v) {        // o16: 16-byte units
-        float4 *dst = reinterpret_cast<float4 *>(vis) + o16;
-        if (a.accumulate) {
-          const float4 old = *dst;
-          v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-        }
-        *dst = v;
-      };
       // block column J of this warp's rows of E -> scratch block k; the column
       // is XORed with the row, so that the row-wise stores and column-wise
       // loads are conflict-free
@@ -203,79 +219,82 @@ __global__ void __launch_bounds__(corrfm::kThreads, 1)
 #pragma unroll
         for (int e = 0; e < 32; ++e) blk[e ^ lane] = ev[e];
       };
-      // outputs (i, j): j the lanes' rows, i the 16 antennas of block row I,
-      // with E of block (I, q) in scratch block k
-      auto conj_block = [&](int I, int k) {
+      // outputs (i, j): j the lanes' rows, i the warp's half (hh) of the 16
+      // antennas of block row I, with E of block (I, q) in scratch block k
+      auto conj_block = [&](int I, int k, const Old &old) {
         const uint32_t *blk = E + k * 1024;
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          uint32_t re[16], er[16];
-          tmem_ld16(trow + 32u * I + 16u * h, re);
-          tmem_ld16(trow + 128u + 32u * I + 16u * h, er);
-          tmem_wait_ld();
+        uint32_t re[16], er[16];
+        tmem_ld16(trow + 32u * I + 16u * hh, re);
+        tmem_ld16(trow + 128u + 32u * I + 16u * hh, er);
+        tmem_wait_ld();
 #pragma unroll
-          for (int ii = 0; ii < 8; ++ii) {
-            const int i = 16 * I + 8 * h + ii;
-            const int n0 = 16 * h + 2 * ii, n1 = n0 + 1;
-            const int32_t en0 = (int32_t)blk[n0 * 32 + (lane ^ n0)];
-            const int32_t en1 = (int32_t)blk[n1 * 32 + (lane ^ n1)];
-            const float x0 = vis_re(re[2 * ii]), y0 = vis_im((int32_t)er[2 * ii] - en0);
-            const float x1 = vis_re(re[2 * ii + 1]), y1 = vis_im((int32_t)er[2 * ii + 1] - en1);
-            // the two pols of j (lanes 2j, 2j + 1): pj = 0 keeps pi = 0 and
-            // sends pi = 1, pj = 1 the reverse, so each writes 16 bytes
-            const float sx = __shfl_xor_sync(0xffffffffu, pj ? x0 : x1, 1);
-            const float sy = __shfl_xor_sync(0xffffffffu, pj ? y0 : y1, 1);
-            if (j <= i)
-              put(2 * ((int64_t)(i * (i + 1) / 2) + j) + pj,
-                  pj ? make_float4(sx, sy, x1, y1) : make_float4(x0, y0, sx, sy));
+        for (int ii = 0; ii < 8; ++ii) {
+          const int i = 16 * I + 8 * hh + ii;
+          const int n0 = 16 * hh + 2 * ii, n1 = n0 + 1;
+          const int32_t en0 = (int32_t)blk[n0 * 32 + (lane ^ n0)];
+          const int32_t en1 = (int32_t)blk[n1 * 32 + (lane ^ n1)];
+          const float x0 = vis_re(re[2 * ii]), y0 = vis_im((int32_t)er[2 * ii] - en0);
+          const float x1 = vis_re(re[2 * ii + 1]), y1 = vis_im((int32_t)er[2 * ii + 1] - en1);
+          // the two pols of j (lanes 2j, 2j + 1): pj = 0 keeps pi = 0 and
+          // sends pi = 1, pj = 1 the reverse, so each writes 16 bytes
+          const float sx = __shfl_xor_sync(0xffffffffu, pj ? x0 : x1, 1);
+          const float sy = __shfl_xor_sync(0xffffffffu, pj ? y0 : y1, 1);
+          float4 v = pj ? make_float4(sx, sy, x1, y1) : make_float4(x0, y0, sx, sy);
+          if (j <= i) {
+            if constexpr (kAcc) v = add4(v, old[ii]);
+            out[i * (i + 1) + 2 * j + pj] = v;
           }
         }
       };
-      // Two rounds, no warp with more than two blocks and then one:
+      // Two rounds, no quarter with more than two blocks and then one:
       //   (0,0) (1,0) | (1,1) (2,1) | (2,2) | (3,3), then
       //   (2,0)       | (3,1)       | (3,2) | (3,0) in row order.
       // Scratch blocks of the first: E (q,q) in q, (1,0) in 4, (2,1) in 5.
       if (ok) {
-        save(q, q);
-        if (q == 1 || q == 2) save(q - 1, 3 + q);
+        if (hh == 0) save(q, q);
+        else if (q == 1 || q == 2) save(q - 1, 3 + q);
       }
       named_bar(1, 32 * kEpiWarps);
       if (ok) {
-        conj_block(q, q);
-        if (q < 2) conj_block(q + 1, 4 + q);
+        if (q < 2) load_old(q + 1, ob);
+        conj_block(q, q, oa);
+        if (q < 2) conj_block(q + 1, 4 + q, ob);
+      }
+      float4 *const row = out + j * (j + 1) + 16 * hh + pj;   // quarter 3: row antenna `j`, eight columns
+      if constexpr (kAcc) {
+        if (q < 3) {
+          load_old(q == 0 ? 2 : 3, oa);
+        } else {
+#pragma unroll
+          for (int jj = 0; jj < 8; ++jj) oa[jj] = row[2 * jj];
+        }
       }
       named_bar(1, 32 * kEpiWarps);
       // the second: (2,0) in 0, (3,1) in 1, (3,2) in 2, (0,3) in 3
       if (ok) {
-        if (q == 0) save(3, 3);
-        if (q == 2) save(0, 0);
-        if (q == 3) {
-          save(1, 1);
-          save(2, 2);
-        }
+        if (q == 0 && hh == 0) save(3, 3);
+        if (q == 2 && hh == 0) save(0, 0);
+        if (q == 3) save(1 + hh, 1 + hh);
       }
       named_bar(1, 32 * kEpiWarps);
       if (ok) {
         if (q < 3) {
-          conj_block(q == 0 ? 2 : 3, q);
-        } else {   // i = 48..63 (this warp's rows), j = 0..15
-          const int64_t tri = (int64_t)(j * (j + 1) / 2);   // (j: the row antenna i here)
+          conj_block(q == 0 ? 2 : 3, q, oa);
+        } else {   // i = 48..63 (this warp's rows; `j` is that antenna), eight j of 0..15
           const uint32_t *blk = E + 3 * 1024;
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h) {
-            uint32_t re[16], er[16];
-            tmem_ld16(trow + 16u * h, re);
-            tmem_ld16(trow + 128u + 16u * h, er);
-            tmem_wait_ld();
+          uint32_t re[16], er[16];
+          tmem_ld16(trow + 16u * hh, re);
+          tmem_ld16(trow + 128u + 16u * hh, er);
+          tmem_wait_ld();
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
-              const int n0 = 16 * h + 2 * jj, n1 = n0 + 1;
-              const int32_t e0 = (int32_t)blk[n0 * 32 + (lane ^ n0)];
-              const int32_t e1 = (int32_t)blk[n1 * 32 + (lane ^ n1)];
-              put(2 * (tri + 8 * h + jj) + pj,
-                  make_float4(vis_re(re[2 * jj]), vis_im(e0 - (int32_t)er[2 * jj]),
-                              vis_re(re[2 * jj + 1]), vis_im(e1 - (int32_t)er[2 * jj + 1])));
-            }
+          for (int jj = 0; jj < 8; ++jj) {
+            const int n0 = 16 * hh + 2 * jj, n1 = n0 + 1;
+            const int32_t e0 = (int32_t)blk[n0 * 32 + (lane ^ n0)];
+            const int32_t e1 = (int32_t)blk[n1 * 32 + (lane ^ n1)];
+            float4 v = make_float4(vis_re(re[2 * jj]), vis_im(e0 - (int32_t)er[2 * jj]),
+                                   vis_re(re[2 * jj + 1]), vis_im(e1 - (int32_t)er[2 * jj + 1]));
+            if constexpr (kAcc) v = add4(v, oa[jj]);
+            row[2 * jj] = v;
           }
         }
       }
@@ -378,8 +397,9 @@ int launch_correlate_freq(const CorrArgs &a, size_t pkt_stride, size_t freq_stri
          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return -2;
-  static SmemAttrOnce attr;
-  if (smem_attr_once(attr, corr_fm_kernel, corrfm::kSmem) != cudaSuccess) return -2;
+  static SmemAttrOnce attr[2];
+  auto kernel = a.accumulate ? corr_fm_kernel<true> : corr_fm_kernel<false>;
+  if (smem_attr_once(attr[a.accumulate ? 1 : 0], kernel, corrfm::kSmem) != cudaSuccess) return -2;
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1)
@@ -388,7 +408,7 @@ int launch_correlate_freq(const CorrArgs &a, size_t pkt_stride, size_t freq_stri
   // CTAs of six)
   const int nfreq = 2 * a.nchan, per = (nfreq + nsm - 1) / nsm;
   const unsigned grid = (unsigned)((nfreq + per - 1) / per);
-  corr_fm_kernel<<<grid, corrfm::kThreads, corrfm::kSmem, st>>>(tmap, a);
+  kernel<<<grid, corrfm::kThreads, corrfm::kSmem, st>>>(tmap, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
