@@ -110,7 +110,7 @@ __device__ void flag_total_power(const FlagArgs &a);
 // ---------------------------------------------------------------- statistics
 // One CTA per (channel slab of up to kFlagSlab channels, time chunk, beam).
 // A warp takes whole TBIN bins of the chunk (every eighth one), or, where the
-// chunk has fewer than eight, an eighth of each.  Its rows come as TMA boxes
+// chunk has fewer than eight long ones, an eighth of each.  Its rows come as TMA boxes
 // of kBatch passes ([rows][min(nchan, 128) channels], channels past nchan
 // zero) into a ring of its own, a.ring - 1 boxes ahead, on its own mbarriers
 // (bounded waits, a.wait_limit_ns, recorded in a.err); a pass is as many
@@ -458,13 +458,25 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
   // warp; the bin's sums combined by the CTA); then the rows beyond the last
   // whole bin: everything but the bins.  (One loop, so that the row code exists
   // once.)
-  const bool by_warp = bin1 - bin0 >= kWarps;
+  // (Split bins go one after the other, each about 2 us of latency and barriers
+  // however short, against 0.4 us per box: from 4 boxes of a single bin to 256
+  // of seven, a warp per bin is no slower.)
+  const bool by_warp = bin1 - bin0 >= kWarps || (TB + brows - 1) / brows <= 2 << (bin1 - bin0);
   const int nbseg = by_warp ? 1 : bin1 - bin0;
-  const int nseg = nbseg + (chunk == a.nchunk - 1 && nbins * TB < T ? 1 : 0);
+  const int ntail = chunk == a.nchunk - 1 ? T - nbins * TB : 0;
+  // a short tail goes to a warp that has no bin
+  const bool tail_in = by_warp && bin1 - bin0 < kWarps && ntail > 0 && ntail <= 2 * brows;
+  const int nseg = nbseg + (ntail > 0 && !tail_in ? 1 : 0);
 #pragma unroll 1
   for (int seg = 0; seg < nseg; ++seg) {
     const bool tail = seg == nbseg, whole = by_warp && !tail;
     int t0 = (bin0 + warp) * TB, n = TB, count = (bin1 - bin0 - warp + kWarps - 1) / kWarps;
+    const bool my_tail = whole && tail_in && warp == bin1 - bin0;
+    if (my_tail) {
+      t0 = nbins * TB;
+      n = ntail;
+      count = 1;
+    }
     if (!whole) {
       const int s0 = tail ? nbins * TB : (bin0 + seg) * TB, len = tail ? T - s0 : TB;
       const int unit = kPix ? a.tds : rpw;
@@ -479,7 +491,7 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const Acc t = bin_total(j);
-          if (lead) {
+          if (lead && !my_tail) {
             Acc *e = sm_bx + 2 * warp * cs + 4 * g + j;
             e[0] = max(e[0], t);
             e[cs] = min(e[cs], t);
@@ -1315,80 +1327,6 @@ int launch_flag_baseline(const float *hist_spec, const float *hist_var, int nave
 }  // namespace dsax
 
 namespace dsax {
-// ---------------------------------------------------------------- decisions
-// Lower median sorted[(n+1)/2 - 1] of v[0..n) in shared memory, by rank
-// counting with ties broken by index (the element a stable sort would put
-// at that position has the same value).  All threads of the block call it.
-__device__ float block_lower_median(const float *v, int n, float *result_slot) {
-  const int k = (n + 1) / 2 - 1;
-  // gs threads (a power of two <= 32) share one element's count
-  int gs = 1;
-  while (gs < 32 && gs * 2 * n <= (int)blockDim.x) gs *= 2;
-  const int sub = threadIdx.x & (gs - 1);
-  const int per = (n + gs - 1) / gs;
-  const int rounds = (n * gs + blockDim.x - 1) / blockDim.x;   // uniform trip count
-  for (int rd = 0; rd < rounds; ++rd) {
-    const int i = (rd * (int)blockDim.x + (int)threadIdx.x) / gs;
-    const bool live = i < n;
-    const float x = live ? v[i] : 0.0f;
-    int r = 0;
-    if (live) {
-      const int j0 = sub * per, j1 = min(n, j0 + per);
-#pragma unroll 8
-      for (int j = j0; j < j1; ++j) {
-        const float y = v[j];
-        r += (y < x) || (y == x && j < i);
-      }
-    }
-    for (int o = gs >> 1; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    if (live && sub == 0 && r == k) *result_slot = x;
-  }
-  __syncthreads();
-  const float med = *result_slot;
-  __syncthreads();
-  return med;
-}
-
-// corr[j - G] = sb[j] - lower median of sb[w0 .. w0 + F), w0 = j, or
-// C - G - F for the last windows (channflag's forward detrend), for j in
-// [G, C - G); one thread per (channel, window element) rank count.
-__device__ void window_detrend(const float *sb, const FlagArgs &a, float *corr) {
-  const int C = a.nchan, G = a.guard, F = a.filt, n = C - 2 * G;
-  const int k = (F + 1) / 2 - 1;
-  for (int idx = threadIdx.x; idx < n * F; idx += blockDim.x) {
-    const int jj = idx / F, i = idx - jj * F;
-    const int j = G + jj;
-    const int w0 = (C - G - j >= F) ? j : C - G - F;
-    const float x = sb[w0 + i];
-    int r = 0;
-    for (int q = 0; q < F; ++q) {
-      const float y = sb[w0 + q];
-      r += (y < x) || (y == x && q < i);
-    }
-    if (r == k) corr[jj] = sb[j] - x;
-  }
-  __syncthreads();
-}
-
-// channflag()'s test statistic as a number: corr[j] / (thr * MAD), so the
-// channel is flagged exactly when |z| > 1 (z = +-1e6 when the MAD is 0 and
-// corr is not; 0 in the guard band).  Used as a learned-flagger feature.
-__device__ void channflag_z(const float *sb, float thr, const FlagArgs &a, float *zout,
-                            float *corr, float *tmp, float *slot) {
-  const int C = a.nchan, G = a.guard, n = C - 2 * G;
-  for (int j = threadIdx.x; j < C; j += blockDim.x) zout[j] = 0.0f;
-  window_detrend(sb, a, corr);
-  const float med = block_lower_median(corr, n, slot);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[i] = fabsf(corr[i] - med);
-  __syncthreads();
-  const float mad = block_lower_median(tmp, n, slot);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const float v = corr[i];
-    zout[G + i] = mad > 0.0f ? v / (thr * mad) : (v > 0.0f ? 1e6f : (v < 0.0f ? -1e6f : 0.0f));
-  }
-  __syncthreads();
-}
-
 __device__ __forceinline__ float slogf(float v) { return copysignf(log1pf(fabsf(v)), v); }
 
 // Learned-flagger input features of one beam (one CTA per beam) from the
@@ -1408,57 +1346,75 @@ __global__ void __launch_bounds__(2 * flag::kDecThreads) lf_stat_features_kernel
   const int b = blockIdx.x;
   const int C = a.nchan, G = a.guard, T = a.ntime, n = C - 2 * G, tds = a.tds, H = T / tds;
   extern __shared__ float lsh[];
-  float *spec = lsh;                                   // C
-  float *corr = spec + C;                              // C
-  float *tmp = corr + C;                               // max(C, ts_base)
-  float *z = tmp + (a.ts_base > C ? a.ts_base : C);    // [4][C]
-  float *zt = z + 4 * C;                               // T
+  float *dsh = lsh;                                    // [4 tests][3][C]: statistic, detrended, scratch
+  float *z = dsh + 12 * C;                             // [4][C]
+  float *tmp = z + 4 * C;                              // ts_base
+  float *zt = tmp + a.ts_base;                         // T
   float *rmax = zt + T;                                // H
   float *rmean = rmax + H;                             // H
-  __shared__ float slot;
-  __shared__ float mu_sd[2];
+  __shared__ uint32_t hist[5][256], sel[5][2];
+  __shared__ float mu_sd[2], ts_med_mad[2];
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const float *tsb = a.ts + (int64_t)b * T;
 
-  for (int c = threadIdx.x; c < C; c += blockDim.x) spec[c] = a.spec[b * C + c];
+  for (int i = tid; i < 4 * C; i += blockDim.x) {
+    const int k = i / C, c = i - k * C;
+    const float *src = k == 0 ? a.spec : k == 1 ? a.var : k == 2 ? a.maxs : a.pp;
+    dsh[3 * C * k + c] = src[b * C + c];
+    z[i] = 0.0f;
+  }
+  for (int i = tid; i < a.ts_base; i += blockDim.x) zt[i] = tsb[i];
   __syncthreads();
-  channflag_z(spec, a.thresh, a, z, corr, tmp, &slot);
-  for (int c = threadIdx.x; c < C; c += blockDim.x) spec[c] = a.var[b * C + c];
+  grp_detrend3(dsh, a, tid, blockDim.x);
   __syncthreads();
-  channflag_z(spec, a.thresh + a.var_add, a, z + C, corr, tmp, &slot);
-  for (int c = threadIdx.x; c < C; c += blockDim.x) spec[c] = a.maxs[b * C + c];
-  __syncthreads();
-  channflag_z(spec, a.thresh, a, z + 2 * C, corr, tmp, &slot);
-  // simple_channflag(pp): one-sided, FBIN-channel mean against med + Thr/sqrt(FBIN) MAD
-  for (int c = threadIdx.x; c < C; c += blockDim.x) spec[c] = a.pp[b * C + c];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) corr[i] = a.pp[b * C + G + i];
-  __syncthreads();
-  {
-    const float med = block_lower_median(corr, n, &slot);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[i] = fabsf(corr[i] - med);
-    __syncthreads();
-    const float mad = block_lower_median(tmp, n, &slot);
-    const float mythr = a.thresh / sqrtf((float)a.fbin);
-    for (int j = threadIdx.x; j < C; j += blockDim.x) {
-      float zz = 0.0f;
-      if (j >= G && j < C - G - a.fbin) {
-        float vv = 0.0f;
-        for (int k = 0; k < a.fbin; ++k) vv += a.parity ? spec[j] : spec[j + k];
-        vv = vv / (float)a.fbin - med;
-        zz = mad > 0.0f ? vv / (mythr * mad) : (vv > 0.0f ? 1e6f : (vv < 0.0f ? -1e6f : 0.0f));
+  // the four channel tests in four groups of 64 threads and the time series'
+  // median and MAD in the other 256, all at once (one after the other by the
+  // whole CTA, each with its barriers, they were half of this kernel)
+  if (warp < 8) {
+    const int k = warp >> 1, gtid = tid & 63, bid = 1 + k;
+    float *sb = dsh + 3 * C * k, *corr = sb + C, *tm = corr + C;
+    if (k < 3) {
+      // channflag()'s test statistic: corr[j] / (thr * MAD), so the channel is
+      // flagged exactly when |z| > 1 (z = +-1e6 when the MAD is 0 and corr is
+      // not; 0 in the guard band)
+      const float thr = k == 1 ? a.thresh + a.var_add : a.thresh;
+      const float med = grp_select_call(corr, n, (n + 1) / 2 - 1, hist[k], sel[k], gtid, 64, bid);
+      for (int i = gtid; i < n; i += 64) tm[i] = fabsf(corr[i] - med);
+      named_bar(bid, 64);
+      const float mad = grp_select_call(tm, n, (n + 1) / 2 - 1, hist[k], sel[k], gtid, 64, bid);
+      for (int i = gtid; i < n; i += 64) {
+        const float v = corr[i];
+        z[k * C + G + i] = mad > 0.0f ? v / (thr * mad) : (v > 0.0f ? 1e6f : (v < 0.0f ? -1e6f : 0.0f));
       }
-      z[3 * C + j] = zz;
+    } else {
+      // simple_channflag(pp): one-sided, FBIN-channel mean against med + Thr/sqrt(FBIN) MAD
+      const float med = grp_select_call(sb + G, n, (n + 1) / 2 - 1, hist[k], sel[k], gtid, 64, bid);
+      for (int i = gtid; i < n; i += 64) tm[i] = fabsf(sb[G + i] - med);
+      named_bar(bid, 64);
+      const float mad = grp_select_call(tm, n, (n + 1) / 2 - 1, hist[k], sel[k], gtid, 64, bid);
+      const float mythr = a.thresh / sqrtf((float)a.fbin);
+      for (int j = G + gtid; j < C - G - a.fbin; j += 64) {
+        float vv = 0.0f;
+        for (int q = 0; q < a.fbin; ++q) vv += a.parity ? sb[j] : sb[j + q];
+        vv = vv / (float)a.fbin - med;
+        z[3 * C + j] = mad > 0.0f ? vv / (mythr * mad) : (vv > 0.0f ? 1e6f : (vv < 0.0f ? -1e6f : 0.0f));
+      }
+    }
+  } else {   // simple_tsflag: median and MAD over the first ts_base samples
+    const int gtid = tid - 256, gsize = (int)blockDim.x - 256, k = (a.ts_base + 1) / 2 - 1;
+    const float med = grp_select_call(zt, a.ts_base, k, hist[4], sel[4], gtid, gsize, 5);
+    for (int i = gtid; i < a.ts_base; i += gsize) tmp[i] = fabsf(zt[i] - med);
+    named_bar(5, gsize);
+    const float mad = grp_select_call(tmp, a.ts_base, k, hist[4], sel[4], gtid, gsize, 5);
+    if (gtid == 0) {
+      ts_med_mad[0] = med;
+      ts_med_mad[1] = mad;
     }
   }
   __syncthreads();
-  // simple_tsflag: median and MAD over the first ts_base samples
-  const float *tsb = a.ts + (int64_t)b * T;
-  for (int i = threadIdx.x; i < a.ts_base; i += blockDim.x) tmp[i] = tsb[i];
-  __syncthreads();
   {
-    const float med = block_lower_median(tmp, a.ts_base, &slot);
-    for (int i = threadIdx.x; i < a.ts_base; i += blockDim.x) tmp[i] = fabsf(tsb[i] - med);
-    __syncthreads();
-    const float mad = block_lower_median(tmp, a.ts_base, &slot);
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+    const float med = ts_med_mad[0], mad = ts_med_mad[1];
+    for (int t = tid; t < T; t += blockDim.x) {
       const float vv = tsb[t] - med;
       float zz = mad > 0.0f ? vv / (a.ts_thresh * mad) : (vv > 0.0f ? 1e6f : (vv < 0.0f ? -1e6f : 0.0f));
       zt[t] = a.tsflag ? zz : 0.0f;
@@ -1558,11 +1514,12 @@ __global__ void __launch_bounds__(2 * flag::kDecThreads) lf_stat_features_kernel
 int launch_lf_stat_features(const FlagArgs &a, float *F, uint16_t *Fbf, cudaStream_t st) {
   if (!a.pix_sum || a.tds < 1 || a.ntime % a.tds || a.nchan > flag::kLfMaxChan) return -1;
   const int H = a.ntime / a.tds;
-  const size_t sh = sizeof(float) * (2 * a.nchan + (a.ts_base > a.nchan ? a.ts_base : a.nchan) +
-                                     4 * a.nchan + a.ntime + 2 * H);
-  if (sh > 200 * 1024) return -1;
+  if (sizeof(float) * (6 * a.nchan + (a.ts_base > a.nchan ? a.ts_base : a.nchan) + a.ntime + 2 * H) >
+      200 * 1024)
+    return -1;
+  const size_t sh = sizeof(float) * (16 * a.nchan + a.ts_base + a.ntime + 2 * H);
   static SmemAttrOnce attr;
-  if (smem_attr_once(attr, lf_stat_features_kernel, 200 * 1024) != cudaSuccess) return -2;
+  if (smem_attr_once(attr, lf_stat_features_kernel, 210 * 1024) != cudaSuccess) return -2;
   lf_stat_features_kernel<<<a.nbeam, 2 * flag::kDecThreads, sh, st>>>(a, F, Fbf);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
