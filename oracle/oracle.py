@@ -704,7 +704,7 @@ def ref_lib(small: bool = False):
 def ref_available() -> bool:
     if os.path.exists(os.path.join(_HERE, "_ref", "libref.so")):
         return True
-    return os.path.isdir(os.environ.get("DSAX_REFERENCE", "/root/reference"))
+    return os.path.isdir(os.path.join(os.environ.get("DSAX_REFERENCE", "/root/reference"), "src"))
 
 
 # --------------------------------------------------------------------------
