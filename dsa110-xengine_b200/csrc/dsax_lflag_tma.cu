@@ -4,15 +4,18 @@
 // Activations live on the padded grid [B][H+2][W+2][64] (BF16, NHWC) whose
 // border pixels are zero.  On that grid the 3x3 neighbourhood of a run of
 // 128 consecutive pixels p0 .. p0+127 is, for tap (dy, dx), the run starting
-// at p0 + dy (W+2) + dx.  Per kernel row dy one TMA load (tensor map over
-// [npp][64] BF16, 128-byte swizzle) brings the 130-pixel band starting at
-// p0 + dy (W+2) - 1; the three taps dx = -1, 0, 1 are the 128-row windows
-// starting 0, 1 and 2 rows into it, each the K-major A operand of
+// at p0 + dy (W+2) + dx.  So one run of 128 + 2 (W+2) + 2 pixels from p0 -
+// (W+2) - 1 on holds all nine: it comes in two TMA boxes (tensor map over
+// [npp][64] BF16, 128-byte swizzle), and the taps are its 128-row windows
+// starting (dy + 1) (W+2) + dx + 1 rows into it, each the K-major A operand of
 // tcgen05.mma kind::f16 (M = 128 pixels, N = Cout, K = 64 channels).  The
 // 128-byte swizzle follows the shared-memory address, so a window may start
-// at any 128-byte row with the usual descriptor.  Three loads and 36 MMAs
-// per tile, no per-pixel gather, each activation row fetched about three
-// times.  Loads that start before the first or run past the last padded
+// at any 128-byte row with the usual descriptor.  Two loads and 36 MMAs per
+// tile, no per-pixel gather, each activation row fetched about twice.  (One
+// 130-pixel band per kernel row fetched it three times, 1.3 GB through L2 for
+// the two layers of 256 beams x 128 x 48, which took 185 us without any MMA.)
+// Measured on 256 x 4096 x 48: inference 0.542 -> 0.507 ms.
+// Loads that start before the first or run past the last padded
 // pixel read zeros (TMA out-of-bounds fill).  Tiles cover the
 // padded grid; the epilogue writes interior pixels only, so the border stays
 // zero.  A layer with fewer input channels (32) keeps them in the first
@@ -38,16 +41,14 @@ namespace dsax {
 
 namespace lftma {
 constexpr int kThreads = 320;
-constexpr int kBandRows = 130;                    // 128 pixels + one on each side
-constexpr int kBandBytes = kBandRows * 128;       // one band: 130 pixels x 64 BF16
-constexpr int kABytes = 17 * 1024;                // stage: the band, rounded to 1 KB
+constexpr int kBandRows = 130;                    // (layer 1's bands: 128 pixels + one on each side)
+constexpr int kMaxWp = 66;                        // padded row (W <= 64)
+// rows of each of the two boxes of a tile's run: whole 8-row swizzle atoms
+__host__ __device__ constexpr int box_rows(int wp) { return ((128 + 2 * wp + 2 + 1) / 2 + 7) & ~7; }
+constexpr int kABytes = 2 * box_rows(kMaxWp) * 128;   // stage: the run (34 KB)
+constexpr int kStages = 4;                        // as many as fit beside the 72 KB of weights
 constexpr int kTaps = 9;
-constexpr int kBands = 3;
 constexpr int kC = 64;                            // channels per padded pixel
-template <int COUT> constexpr int stages() {
-  return (200 * 1024 - kTaps * COUT * 128) / kABytes < 8 ? (200 * 1024 - kTaps * COUT * 128) / kABytes
-                                                          : 8;
-}
 }  // namespace lftma
 
 struct LfTmaArgs {
@@ -85,7 +86,6 @@ __global__ void __launch_bounds__(lftma::kThreads, 1)
   constexpr int WBYTES = kTaps * COUT * 128;
   constexpr uint32_t IDESC = umma_idesc(/*F32*/ 1, /*BF16*/ 1, /*BF16*/ 1, 128, COUT);
   constexpr uint32_t TCOLS = 2 * COUT;
-  constexpr int kStages = stages<COUT>();
   static_assert(COUT == 64, "64 output channels");
   static_assert(CIN == 32 || CIN == 64, "32 or 64 real input channels");
   constexpr int KK = CIN / 16;   // 16-channel K steps per tap
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(lftma::kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 256);
+      mbar_init(&tempty_bar[b], 8);
     }
     mbar_init(&w_bar, 1);
     mbar_init(&final_bar, 1);
@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(lftma::kThreads, 1)
         }
       }
       tc_fence_before();
-      mbar_arrive(&tempty_bar[bf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[bf]);
       const int pp = ((int)blockIdx.x + i * (int)gridDim.x) * 128 + m;
       if (!ok || pp >= npp) continue;
       const int r = small ? div_small(pp, Wp, iWp) : pp / Wp;
@@ -215,17 +216,18 @@ __global__ void __launch_bounds__(lftma::kThreads, 1)
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tin)) : "memory");
-      const int G = nmine * kBands;
+      const int br = box_rows(Wp);
       int g = 0;
-      for (; g < G && !abort_sh; ++g) {
+      for (; g < nmine && !abort_sh; ++g) {
         const int s = g % kStages;
         if (!mbar_wait_bounded(&empty_bar[s], ((uint32_t)(g / kStages) & 1u) ^ 1u, &abort_sh, a.err,
                                DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
           break;
-        const int i = g / kBands, band = g - i * kBands;   // kernel row dy = band - 1
-        const int row = ((int)blockIdx.x + i * (int)gridDim.x) * 128 + (band - 1) * Wp - 1;
-        mbar_arrive_expect_tx(&full_bar[s], (uint32_t)kBandBytes);
-        tma_load_2d(asm_base + (uint32_t)s * kABytes, &tin, 0, row, &full_bar[s]);
+        const int row = ((int)blockIdx.x + g * (int)gridDim.x) * 128 - Wp - 1;
+        const uint32_t dst = asm_base + (uint32_t)s * kABytes;
+        mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(2 * br * 128));
+        tma_load_2d(dst, &tin, 0, row, &full_bar[s]);
+        tma_load_2d(dst + (uint32_t)br * 128u, &tin, 0, row + br, &full_bar[s]);
       }
       // loads still landing after an abort: wait (bounded) before exiting
       volatile int no_abort = 0;
@@ -257,26 +259,26 @@ __global__ void __launch_bounds__(lftma::kThreads, 1)
         // cannot overflow below 256 KB), so each MMA costs one add and the
         // issue.
         const uint32_t dcol = tmem + (uint32_t)(bf * COUT);
+        const int s = i % kStages;
+        if (!mbar_wait_bounded(&full_bar[s], (uint32_t)(i / kStages) & 1u, &abort_sh, a.err,
+                               DEV_ERR_WAIT_FULL, a.wait_limit_ns)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint64_t ab = adesc0 + (uint64_t)(((uint32_t)s * kABytes) >> 4);
 #pragma unroll
-        for (int band = 0; band < kBands; ++band) {
-          const int g = i * kBands + band, s = g % kStages;
-          if (!mbar_wait_bounded(&full_bar[s], (uint32_t)(g / kStages) & 1u, &abort_sh, a.err,
-                                 DEV_ERR_WAIT_FULL, a.wait_limit_ns)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t ab = adesc0 + (uint64_t)(((uint32_t)s * kABytes) >> 4);
+        for (int dy = 0; dy < 3; ++dy) {
+          const uint64_t aw = ab + (uint64_t)(dy * Wp * 8);   // rows of 128 bytes, in 16-byte units
 #pragma unroll
-          for (int dx = 0; dx < 3; ++dx)   // tap (band, dx): window starting dx rows in
+          for (int dx = 0; dx < 3; ++dx)   // tap (dy, dx): window starting dy Wp + dx rows in
 #pragma unroll
             for (int kk = 0; kk < KK; ++kk)   // K = CIN bf16 = KK x 16
-              umma_f16(dcol, ab + (uint64_t)((128 * dx + 32 * kk) >> 4),
-                       bdesc0 + (uint64_t)(((3 * band + dx) * COUT * 128 + 32 * kk) >> 4), IDESC,
-                       (band | dx | kk) != 0);
-          umma_commit(&empty_bar[s]);
+              umma_f16(dcol, aw + (uint64_t)((128 * dx + 32 * kk) >> 4),
+                       bdesc0 + (uint64_t)(((3 * dy + dx) * COUT * 128 + 32 * kk) >> 4), IDESC,
+                       (dy | dx | kk) != 0);
         }
-        if (!ok) break;
+        umma_commit(&empty_bar[s]);
         umma_commit(&tfull_bar[bf]);
       }
       umma_commit(&final_bar);
@@ -580,15 +582,15 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
 
 namespace {
 
-// Tensor map over a padded grid [npp][ch] BF16 with 130-pixel boxes: ch =
+// Tensor map over a padded grid [npp][ch] BF16 with boxes of `rows` pixels: ch =
 // 64 (128-byte rows, 128-byte swizzle) or 8 (16-byte rows, no swizzle);
 // zero fill out of bounds.
-int encode_grid_map(CUtensorMap *map, const uint16_t *grid, int64_t npp, int ch) {
+int encode_grid_map(CUtensorMap *map, const uint16_t *grid, int64_t npp, int ch, int rows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (!fn || npp < 1 || npp > (int64_t)0x7fffffff || (ch != 64 && ch != 8)) return -1;
   const cuuint64_t dims[2] = {(cuuint64_t)ch, (cuuint64_t)npp};
   const cuuint64_t strides[1] = {(cuuint64_t)ch * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)ch, (cuuint32_t)lftma::kBandRows};
+  const cuuint32_t box[2] = {(cuuint32_t)ch, (cuuint32_t)rows};
   const cuuint32_t estr[2] = {1u, 1u};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(grid), dims,
                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -599,7 +601,7 @@ int encode_grid_map(CUtensorMap *map, const uint16_t *grid, int64_t npp, int ch)
 
 template <int COUT, bool PROJ, int CIN>
 int conv_tma_launch(const CUtensorMap &map, const LfTmaArgs &a, int num_sms, cudaStream_t st) {
-  constexpr int smem = 1024 + lftma::kTaps * COUT * 128 + lftma::stages<COUT>() * lftma::kABytes;
+  constexpr int smem = 1024 + lftma::kTaps * COUT * 128 + lftma::kStages * lftma::kABytes;
   static SmemAttrOnce attr;
   if (smem_attr_once(attr, lf_conv_tma_kernel<COUT, PROJ, CIN>, smem) != cudaSuccess) return -2;
   const int64_t npp = (int64_t)a.B * (a.H + 2) * (a.W + 2);
@@ -640,7 +642,7 @@ int lf_tma_layer1(const LfNet &net, const uint8_t *wimg, const uint16_t *featp, 
   static_assert(kLfCin[0] == 8 && kLfCout[0] == lf1::kCout, "layer 1 is 8 -> 32");
   const int64_t npp = (int64_t)B * (H + 2) * (W + 2);
   CUtensorMap mf;
-  if (encode_grid_map(&mf, featp, npp, 8) != 0) return -1;
+  if (encode_grid_map(&mf, featp, npp, 8, lftma::kBandRows) != 0) return -1;
   static SmemAttrOnce attr;
   if (smem_attr_once(attr, lf_conv1_tma_kernel, lf1::kSmemBytes) != cudaSuccess) return -2;
   Lf1Args a{};
@@ -662,7 +664,10 @@ int lf_tma_layers23(const LfNet &net, const uint8_t *wimg, const uint16_t *act1p
                 "padded layers are written for 32 -> 64 -> 64");
   const int64_t npp = (int64_t)B * (H + 2) * (W + 2);
   CUtensorMap m1, m2;
-  if (encode_grid_map(&m1, act1p, npp, 64) != 0 || encode_grid_map(&m2, act2p, npp, 64) != 0) return -1;
+  if (W + 2 > lftma::kMaxWp) return -1;
+  const int br = lftma::box_rows(W + 2);
+  if (encode_grid_map(&m1, act1p, npp, 64, br) != 0 || encode_grid_map(&m2, act2p, npp, 64, br) != 0)
+    return -1;
   LfTmaArgs a{};
   a.err = err;
   a.B = B; a.H = H; a.W = W;
