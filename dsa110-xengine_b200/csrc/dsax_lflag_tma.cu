@@ -41,7 +41,6 @@ namespace dsax {
 
 namespace lftma {
 constexpr int kThreads = 320;
-constexpr int kBandRows = 130;                    // (layer 1's bands: 128 pixels + one on each side)
 constexpr int kMaxWp = 66;                        // padded row (W <= 64)
 // rows of each of the two boxes of a tile's run: whole 8-row swizzle atoms
 __host__ __device__ constexpr int box_rows(int wp) { return ((128 + 2 * wp + 2 + 1) / 2 + 7) & ~7; }
@@ -338,29 +337,32 @@ __global__ void lf_pad_border_kernel(uint16_t *act, int B, int H, int W, int chu
 
 // ---------------------------------------------------------------------------
 // First layer (8 -> 32 channels) from the zero-bordered feature grid
-// [B][H+2][W+2][8] BF16.  A tap is 16 bytes, too narrow for a swizzled box,
-// so per tile three unswizzled TMA boxes of 130 pixels x 16 B (one per
-// kernel row) land in a band slot, and four builder warps copy each pixel's
-// nine taps into the K-major 128-byte-swizzled A tile (K = 72 in two 64-wide
-// blocks, k = 8 tap + ci; the rest of the second block stays zero), then
-// 5 MMAs of N = 32 (K 64 + 16).  The epilogue writes channels 0-31 of the interior
-// pixels of the 64-channel grid the next layer reads (channels 32-63 are
-// zero there).
-//   warps 0-3 : A-tile builders      warps 4-7 : epilogue
-//   warp  8   : TMA producer         warp  9   : TMEM, weights, UMMA issue
+// [B][H+2][W+2][8] BF16.  A pixel is 16 bytes, so a run of pixels is already
+// a K-major operand without swizzle: eight pixels make one 8 x 16 B core
+// matrix, the next eight lie 128 bytes on, and the descriptor's leading
+// offset is free to point at any other tap as the second half of a K = 16
+// step.  The run of 128 + 2 (W+2) + 2 pixels that holds a tile's nine taps
+// comes in two TMA boxes and feeds the MMAs where it lies: five of N = 32 over
+// taps (0,1) (2,3) (4,5) (6,7) (8, zeros).  The epilogue writes channels 0-31
+// of the interior pixels of the 64-channel grid the next layer reads (channels
+// 32-63 are zero there).
+// Built by four warps into a swizzled A tile instead, the nine 16-byte copies
+// per pixel, two proxy fences and 256 barrier arrivals a tile took most of the
+// time: 74 us on 256 x 128 x 48 pixels, now 62 with one CTA per SM and 50 with
+// two (each waits for loads and TMEM reads of its own; 45 KB, 128 TMEM columns).
+//   warps 0-3, 4-7 : epilogue of even, odd tiles
+//   warp  8        : TMA producer      warp  9   : TMEM, weights, UMMA issue
 namespace lf1 {
 constexpr int kThreads = 320;
-constexpr int kBandPix = 130;
-constexpr int kBandBytes = kBandPix * 16;           // 2,080
-constexpr int kBandStride = 2176;                   // 128-byte aligned band offset
-constexpr int kSlotStride = 6656;                   // 128-byte aligned slot
+constexpr int kSlotBytes = 2 * lftma::box_rows(lftma::kMaxWp) * 16;   // a tile's run of pixels
 constexpr int kSlots = 8;
-constexpr int kABytes = 2 * 16384;                  // two K blocks of 128 x 128 B
-constexpr int kAStages = 4;
+constexpr int kAccum = 4;                           // accumulators: two per epilogue group
 constexpr int kCout = 32;
 constexpr int kWBytes = 2 * kCout * 128;            // B operand: two K blocks
-constexpr int kSmemBytes = 1024 + kWBytes + kAStages * kABytes + kSlots * kSlotStride;
+constexpr int kZeroBytes = 128 * 16;                // the second half of tap 8's step
+constexpr int kSmemBytes = 1024 + kWBytes + kSlots * kSlotBytes + kZeroBytes;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
+static_assert(kSlotBytes % 128 == 0, "TMA destination alignment");
 }  // namespace lf1
 
 struct Lf1Args {
@@ -372,18 +374,16 @@ struct Lf1Args {
   uint64_t wait_limit_ns;
 };
 
-__global__ void __launch_bounds__(lf1::kThreads, 1)
+__global__ void __launch_bounds__(lf1::kThreads, 2)
     lf_conv1_tma_kernel(const __grid_constant__ CUtensorMap tfeat, Lf1Args a) {
   using namespace lf1;
   constexpr uint32_t IDESC = umma_idesc(/*F32*/ 1, /*BF16*/ 1, /*BF16*/ 1, 128, kCout);
-  constexpr uint32_t TCOLS = 2 * kCout;   // 64
+  constexpr uint32_t TCOLS = kAccum * kCout;   // 128
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bfull_bar[kSlots];
   __shared__ __align__(8) uint64_t bempty_bar[kSlots];
-  __shared__ __align__(8) uint64_t afull_bar[kAStages];
-  __shared__ __align__(8) uint64_t aempty_bar[kAStages];
-  __shared__ __align__(8) uint64_t tfull_bar[2];
-  __shared__ __align__(8) uint64_t tempty_bar[2];
+  __shared__ __align__(8) uint64_t tfull_bar[kAccum];
+  __shared__ __align__(8) uint64_t tempty_bar[kAccum];
   __shared__ __align__(8) uint64_t w_bar;
   __shared__ __align__(8) uint64_t final_bar;
   __shared__ uint32_t tmem_base_sh;
@@ -394,15 +394,11 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t *const gbase = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t wsm = base;
-  const uint32_t a_base = base + kWBytes;                    // 1024-aligned (kWBytes = 8 KB)
-  const uint32_t b_base = a_base + kAStages * kABytes;
+  const uint32_t b_base = base + kWBytes;
+  const uint32_t z_base = b_base + kSlots * kSlotBytes;
   for (int i = tid; i < kCout; i += blockDim.x) s_bias[i] = a.bias[i];
-  // chunks 1-7 of every A stage's second K block are never written again
-  for (int i = tid; i < kAStages * 128 * 7; i += blockDim.x) {
-    const int st = i / (128 * 7), r = (i / 7) % 128, ch = 1 + i % 7;
-    *reinterpret_cast<uint4 *>(gbase + kWBytes + st * kABytes + 16384 + sw128_offset(r, ch)) =
-        make_uint4(0u, 0u, 0u, 0u);
-  }
+  for (int i = tid; i < kZeroBytes / 16; i += blockDim.x)
+    reinterpret_cast<uint4 *>(gbase + (z_base - base))[i] = make_uint4(0u, 0u, 0u, 0u);
   fence_proxy_async_smem();
 
   const int Hp = a.H + 2, Wp = a.W + 2;
@@ -413,15 +409,11 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
   if (tid == 0) {
     for (int r = 0; r < kSlots; ++r) {
       mbar_init(&bfull_bar[r], 1);
-      mbar_init(&bempty_bar[r], 128);
+      mbar_init(&bempty_bar[r], 1);
     }
-    for (int s2 = 0; s2 < kAStages; ++s2) {
-      mbar_init(&afull_bar[s2], 128);
-      mbar_init(&aempty_bar[s2], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kAccum; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], 128);
+      mbar_init(&tempty_bar[b], 4);
     }
     mbar_init(&w_bar, 1);
     mbar_init(&final_bar, 1);
@@ -437,42 +429,15 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
   tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
 
-  if (warp < 4) {
-    // ------------------------------------------------------------ A builders
-    const int m = tid;
-    for (int i = 0; i < nmine && !abort_sh; ++i) {
-      const int r = i % kSlots, s2 = i % kAStages;
-      if (!mbar_wait_bounded(&bfull_bar[r], (uint32_t)(i / kSlots) & 1u, &abort_sh, a.err,
-                             DEV_ERR_WAIT_FULL, a.wait_limit_ns))
-        break;
-      uint4 t[9];
-      const uint8_t *slot = gbase + kWBytes + kAStages * kABytes + r * kSlotStride;
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap)
-        t[tap] = *reinterpret_cast<const uint4 *>(slot + (tap / 3) * kBandStride + (m + tap % 3) * 16);
-      // the next TMA load (async proxy) overwrites this slot: order the reads
-      fence_proxy_async_smem();
-      mbar_arrive(&bempty_bar[r]);
-      if (!mbar_wait_bounded(&aempty_bar[s2], ((uint32_t)(i / kAStages) & 1u) ^ 1u, &abort_sh, a.err,
-                             DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
-        break;
-      uint8_t *as = gbase + kWBytes + s2 * kABytes;
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap)
-        *reinterpret_cast<uint4 *>(as + (tap / 8) * 16384 + sw128_offset((uint32_t)m, (uint32_t)(tap % 8))) =
-            t[tap];
-      fence_proxy_async_smem();
-      mbar_arrive(&afull_bar[s2]);
-    }
-  } else if (warp < 8) {
+  if (warp < 8) {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;
     const int m = 32 * q + lane;
     const bool small = npp < (1 << 24);
     const float iWp = 1.0f / (float)Wp, iHp = 1.0f / (float)Hp;
-    for (int i = 0; i < nmine; ++i) {
-      const int bf = i & 1;
-      bool ok = mbar_wait_bounded(&tfull_bar[bf], (uint32_t)(i >> 1) & 1u, &abort_sh, a.err,
+    for (int i = warp >> 2; i < nmine; i += 2) {
+      const int bf = i % kAccum;
+      bool ok = mbar_wait_bounded(&tfull_bar[bf], (uint32_t)(i / kAccum) & 1u, &abort_sh, a.err,
                                   DEV_ERR_WAIT_ACCUM, a.wait_limit_ns);
       tc_fence_after();
       ok = __all_sync(0xffffffffu, ok && !abort_sh);
@@ -485,7 +450,8 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
         for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(rr[e]);
       }
       tc_fence_before();
-      mbar_arrive(&tempty_bar[bf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty_bar[bf]);
       const int pp = ((int)blockIdx.x + i * (int)gridDim.x) * 128 + m;
       if (!ok || pp >= npp) continue;
       const int r = small ? div_small(pp, Wp, iWp) : pp / Wp;
@@ -507,18 +473,18 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tfeat)) : "memory");
+      const int br = lftma::box_rows(Wp);
       int i = 0;
       for (; i < nmine && !abort_sh; ++i) {
         const int r = i % kSlots;
         if (!mbar_wait_bounded(&bempty_bar[r], ((uint32_t)(i / kSlots) & 1u) ^ 1u, &abort_sh, a.err,
                                DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
           break;
-        const int p0 = ((int)blockIdx.x + i * (int)gridDim.x) * 128;
-        mbar_arrive_expect_tx(&bfull_bar[r], (uint32_t)(3 * kBandBytes));
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
-          tma_load_2d(b_base + (uint32_t)(r * kSlotStride + dy * kBandStride), &tfeat, 0,
-                      p0 + (dy - 1) * Wp - 1, &bfull_bar[r]);
+        const int p0 = ((int)blockIdx.x + i * (int)gridDim.x) * 128 - Wp - 1;
+        const uint32_t dst = b_base + (uint32_t)(r * kSlotBytes);
+        mbar_arrive_expect_tx(&bfull_bar[r], (uint32_t)(2 * br * 16));
+        tma_load_2d(dst, &tfeat, 0, p0, &bfull_bar[r]);
+        tma_load_2d(dst + (uint32_t)(br * 16), &tfeat, 0, p0 + br, &bfull_bar[r]);
       }
       // loads still landing after an abort: wait (bounded) before exiting
       volatile int no_abort = 0;
@@ -533,7 +499,6 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
     if (lane == 0) {
       mbar_arrive_expect_tx(&w_bar, (uint32_t)kWBytes);
       bulk_g2s(wsm, a.wimg, (uint32_t)kWBytes, &w_bar);
-      const uint64_t adesc0 = umma_desc_sw128(a_base, 1024u);
       const uint64_t bdesc0 = umma_desc_sw128(wsm, 1024u);
       bool ok = mbar_wait_bounded(&w_bar, 0u, &abort_sh, a.err, DEV_ERR_WAIT_FULL, a.wait_limit_ns);
       if (!ok) {   // the weight copy may still be landing
@@ -541,25 +506,27 @@ __global__ void __launch_bounds__(lf1::kThreads, 1)
         mbar_wait_bounded(&w_bar, 0u, &no_abort, a.err, DEV_ERR_WAIT_FULL, drain_limit(a.wait_limit_ns));
       }
       for (int i = 0; i < nmine && ok && !abort_sh; ++i) {
-        const int bf = i & 1, s2 = i % kAStages;
-        if (!mbar_wait_bounded(&tempty_bar[bf], ((uint32_t)(i >> 1) & 1u) ^ 1u, &abort_sh, a.err,
+        const int bf = i % kAccum, r = i % kSlots;
+        if (!mbar_wait_bounded(&tempty_bar[bf], ((uint32_t)(i / kAccum) & 1u) ^ 1u, &abort_sh, a.err,
                                DEV_ERR_WAIT_EMPTY, a.wait_limit_ns))
           break;
-        if (!mbar_wait_bounded(&afull_bar[s2], (uint32_t)(i / kAStages) & 1u, &abort_sh, a.err,
+        if (!mbar_wait_bounded(&bfull_bar[r], (uint32_t)(i / kSlots) & 1u, &abort_sh, a.err,
                                DEV_ERR_WAIT_FULL, a.wait_limit_ns))
           break;
         tc_fence_after();
-        const uint64_t ab = adesc0 + (uint64_t)(((uint32_t)s2 * kABytes) >> 4);
+        const uint32_t ab = b_base + (uint32_t)(r * kSlotBytes);
         const uint32_t dcol = tmem + (uint32_t)(bf * kCout);
-        // K = 72: block 0 holds taps 0-7, block 1 tap 8 in its first 16
-        // K elements (the rest is zero and not issued)
+        // K = 72: the weights' block 0 holds taps 0-7, block 1 tap 8 in its
+        // first 8 K elements and zeros in the next 8
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-          for (int kk = 0; kk < (kb == 0 ? 4 : 1); ++kk)
-            umma_f16(dcol, ab + (uint64_t)((kb * 16384 + 32 * kk) >> 4),
-                     bdesc0 + (uint64_t)((kb * kCout * 128 + 32 * kk) >> 4), IDESC, (kb | kk) != 0);
-        umma_commit(&aempty_bar[s2]);
+        for (int kk = 0; kk < 5; ++kk) {
+          const int t0 = 2 * kk, t1 = t0 + 1;
+          const uint32_t s0 = ab + (uint32_t)((t0 / 3 * Wp + t0 % 3) * 16);
+          const uint32_t s1 = kk < 4 ? ab + (uint32_t)((t1 / 3 * Wp + t1 % 3) * 16) : z_base;
+          umma_f16(dcol, umma_desc_plain(s0, s1 - s0, 128u),
+                   bdesc0 + (uint64_t)(((kk / 4) * kCout * 128 + 32 * (kk % 4)) >> 4), IDESC, kk != 0);
+        }
+        umma_commit(&bempty_bar[r]);
         umma_commit(&tfull_bar[bf]);
       }
       umma_commit(&final_bar);
@@ -642,14 +609,15 @@ int lf_tma_layer1(const LfNet &net, const uint8_t *wimg, const uint16_t *featp, 
   static_assert(kLfCin[0] == 8 && kLfCout[0] == lf1::kCout, "layer 1 is 8 -> 32");
   const int64_t npp = (int64_t)B * (H + 2) * (W + 2);
   CUtensorMap mf;
-  if (encode_grid_map(&mf, featp, npp, 8, lftma::kBandRows) != 0) return -1;
+  if (W + 2 > lftma::kMaxWp ||
+      encode_grid_map(&mf, featp, npp, 8, lftma::box_rows(W + 2)) != 0) return -1;
   static SmemAttrOnce attr;
   if (smem_attr_once(attr, lf_conv1_tma_kernel, lf1::kSmemBytes) != cudaSuccess) return -2;
   Lf1Args a{};
   a.wimg = wimg; a.bias = net.b[0]; a.out = act1p; a.err = err;
   a.B = B; a.H = H; a.W = W; a.wait_limit_ns = wait_limit_ns;
   const int ntiles = (int)((npp + 127) / 128);
-  const int grid = ntiles < num_sms ? ntiles : num_sms;
+  const int grid = ntiles < 2 * num_sms ? ntiles : 2 * num_sms;   // two CTAs per SM
   if (grid < 1) return 0;
   lf_conv1_tma_kernel<<<grid, lf1::kThreads, lf1::kSmemBytes, st>>>(mf, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

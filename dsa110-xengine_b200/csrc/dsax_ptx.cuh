@@ -204,6 +204,17 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t sbo
   return d;
 }
 
+// K-major operand without swizzle: core matrices of 8 rows x 16 bytes (128 B,
+// contiguous); `lbo` steps to the next 16 bytes of K, `sbo` to the next 8 rows.
+__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)1u << 46;
+  return d;
+}
+
 // MN-major operand (the M / N index contiguous) in the 128-byte-swizzle
 // layout: atoms of 8 K rows x 128 bytes of M / N (1024 B); `lbo` steps to the
 // next 128 bytes of M / N, `sbo` to the next 8 K rows.
