@@ -736,8 +736,11 @@ def main():
     kernel_ms = {}
     if cfg.corr_path != 1:
         reo = torch.empty(2048 * 768 * 64 * 2, dtype=torch.uint8, device=f"cuda:{dev}")
-        tfmt = dsax.FMT_REORDERED if cfg.corr_path == 2 else dsax.FMT_CHANMAJOR
-        names = (("reorder_kernel", "corr_kernel") if cfg.corr_path == 2
+        # (paths 0 and 4 turn to one stream per frequency: the same two kernels
+        # with other strides, reached here through the REORDER-key format)
+        rows = cfg.corr_path in (0, 2, 4)
+        tfmt = dsax.FMT_REORDERED if rows else dsax.FMT_CHANMAJOR
+        names = (("reorder_kernel", "corr_fm_kernel") if rows
                  else ("reorder_cm_kernel", "corr_cm_kernel"))
         for name, fn in ((names[0], lambda s: ctx.corner_turn(ins[s % nbuf], reo, tfmt)),
                          (names[1], lambda s: ctx.correlate(reo, vis, fmt=tfmt))):
@@ -821,10 +824,10 @@ def main():
             "config": {"workload": "full-size correlator block [2048][63->64][384][2][2] "
                                    "-> xGPU triangular 768x2080x4 complex FP32",
                        "block_bytes": BLOCK_IN, "vis_bytes": VIS_OUT,
-                       "corr_path": ["channel-major corner turn + bulk-fed correlate", "fused",
+                       "corr_path": ["corner turn to frequency streams + correlate", "fused",
                                      "REORDER-layout corner turn + correlate",
                                      "channel-major corner turn + directly fed correlate",
-                                     "channel-major corner turn + bulk-fed correlate",
+                                     "corner turn to frequency streams + correlate",
                                      "channel-major corner turn + bulk-fed correlate, 16 unpack warps",
                                      "captured block read directly (4-CTA clusters, no corner turn)",
                                      "captured block read directly (4-CTA clusters), 16 unpack warps"
