@@ -123,9 +123,11 @@ __device__ void flag_total_power(const FlagArgs &a);
 // uint8 the 128-byte slab rows in and out (about 3.6 TB/s), in 1.7 waves of
 // CTAs.
 //
-// Sums are FP64 for FP32 data and exact 32-bit integers for uint8 (a lane
-// takes at most a quarter of the rows, so 255^2 products stay below 2^32; the
-// launcher checks it).  Four rows of uint8 are transposed to words of one
+// Sums are FP64 for FP32 data and exact integers for uint8: 32 bits within a
+// range of rows (a lane's share of a bin or of the tail is at most 49,152 rows
+// of an accepted block, so the 255^2 products stay below 2^32; flag_shape_ok),
+// 64 bits for the squares from there on, since a lane may have several bins.
+// Four rows of uint8 are transposed to words of one
 // channel, whose sum and sum of squares are one dp4a each.  A lane's sums are
 // combined with the other row phases' in a fixed order, and the chunks' by the
 // chunk CTA that finishes last, in chunk order, so results do not depend on
@@ -224,12 +226,14 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
   }
   __syncthreads();
 
-  Acc s[4], q[4], bs[4];                       // sums, squares, sums of the current bin
+  using Sq = typename std::conditional<kU8, unsigned long long, double>::type;
+  Acc s[4], q[4], bs[4];                       // sums, squares (uint8: of the current range), sums of the current bin
+  Sq sq[4];                                    // uint8: squares of the earlier ranges
   float m[4];                                  // maxima (uint8: in mx)
   uint32_t mx[2] = {0u, 0u};                   // uint8 maxima of channels 0, 2 and 1, 3
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    s[j] = 0; q[j] = 0; bs[j] = 0;
+    s[j] = 0; q[j] = 0; bs[j] = 0; sq[j] = 0;
     m[j] = -INFINITY;
   }
   // the running pixel of channels lane, lane + 32, ... (sum and maximum over
@@ -487,6 +491,13 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
       count = 1;
     }
     run(t0, n, kWarps * TB, count, [&]() {
+      if constexpr (kU8) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sq[j] += q[j];
+          q[j] = 0;
+        }
+      }
       if (whole) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -533,7 +544,7 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const double mj = kU8 ? (double)((mx[j & 1] >> (8 * (j & 2))) & 0xFFFFu) : (double)m[j];
-        sm_part[(warp * rpw + rp) * cs + 4 * g + j] = pass == 0 ? (double)s[j] : pass == 1 ? (double)q[j] : mj;
+        sm_part[(warp * rpw + rp) * cs + 4 * g + j] = pass == 0 ? (double)s[j] : pass == 1 ? (double)(kU8 ? sq[j] : (Sq)q[j]) : mj;
       }
     }
     __syncthreads();
@@ -1159,8 +1170,11 @@ bool flag_shape_ok(const FlagArgs &a) {
   if (a.pix_sum && (u8 || a.nchan > kFlagSlab || a.tds < 1 || a.tbin % a.tds ||
                     a.ntime % a.tbin || a.tds > 256 || (size_t)a.tds * a.nchan * 4 > 24576))
     return false;
-  // uint8 sums are 32-bit: a lane's share of the rows, as before at most
-  // 32768 of an eighth (more in the narrowest slabs, whose passes hold more rows)
+  // uint8 sums are 32-bit within a range of rows (a bin, where there are at
+  // least eight of them or they are short; else a warp's eighth of a bin or of
+  // the tail).  A slab of g groups takes 32,768 * (256 / g) rows, an eighth of
+  // them in passes of 32 / g rows: at most 49,152 rows per lane (20 groups)
+  // where 2^32 / 255^2 is 66,051.
   const int cs = a.nchan < kFlagSlab ? a.nchan : kFlagSlab;
   const int P = flag::kStatThreads / (cs / 4);
   if (u8 && (a.ntime + P - 1) / P > 32768) return false;
