@@ -153,7 +153,7 @@ extern "C" int dsax_agc_enable(dsax_ctx *c, int mode) {
                                           up256(sizeof(AgcHdr)));
   agc_reset_kernel<<<16, 256, 0, c->stream>>>(h, mode == 1 ? 1 : 0, nbeam, rest,
                                              (kAgcNbp + 2) * nbeam);
-  if (cudaGetLastError() != cudaSuccess) return cuda_check(c, cudaGetLastError(), "AGC reset");
+  if (cudaGetLastError() != cudaSuccess) return launch_failed(c, "AGC reset");
   c->agc_on = 1;
   return DSAX_OK;
 }

@@ -31,6 +31,12 @@ int cuda_check(dsax_ctx *c, cudaError_t e, const char *what) {
   return set_error(c, DSAX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+int launch_failed(dsax_ctx *c, const char *what) {
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_check(c, e, what);
+  return set_error(c, DSAX_ERR_CUDA, "%s: refused or failed", what);
+}
+
 // Makes the context's device current for the duration of a call.
 DeviceGuard::DeviceGuard(int dev) {
   cudaGetDevice(&prev_);
@@ -234,13 +240,13 @@ static int correlate_device(dsax_ctx *c, int fmt, const void *in, float *vis, in
   if (fmt == DSAX_FMT_CHANMAJOR) {
     a.nant_in = 64;
     if (launch_correlate_chanmajor(a, c->stream, c->cfg.corr_path) != 0)
-      return cuda_check(c, cudaGetLastError(), "correlator launch");
+      return launch_failed(c, "correlator launch");
     return DSAX_OK;
   }
   if (fmt == DSAX_FMT_CAPTURED && corr_path_fused(c->cfg.corr_path) && captured_cluster_ok(a)) {
     // the correlator reads the captured block directly (no corner turn)
     if (launch_correlate_captured_cluster(a, c->stream, corr_path_unpack_warps(c->cfg.corr_path)) != 0)
-      return cuda_check(c, cudaGetLastError(), "correlator launch");
+      return launch_failed(c, "correlator launch");
     return DSAX_OK;
   }
   if (fmt == DSAX_FMT_CAPTURED && c->cfg.corr_path != 1) {
@@ -251,23 +257,23 @@ static int correlate_device(dsax_ctx *c, int fmt, const void *in, float *vis, in
     uint8_t *tmp = static_cast<uint8_t *>(c->aux[AUX_REORDERED].ptr);
     if (c->cfg.corr_path == 2) {   // REORDER-key layout (massage) + row loads
       if (launch_reorder(a.in, tmp, c->cfg.npkt, c->cfg.nant_in, c->cfg.nchan, c->stream) != 0)
-        return cuda_check(c, cudaGetLastError(), "corner-turn launch");
+        return launch_failed(c, "corner-turn launch");
       a.in = tmp;
       a.nant_in = 64;
       fmt = DSAX_FMT_REORDERED;
     } else {                       // channel (3, 5) or frequency streams
       if (launch_corner_turn(a.in, tmp, c->cfg.npkt, c->cfg.nant_in, c->cfg.nchan, c->stream,
                              c->cfg.corr_path) != 0)
-        return cuda_check(c, cudaGetLastError(), "corner-turn launch");
+        return launch_failed(c, "corner-turn launch");
       a.in = tmp;
       a.nant_in = 64;
       if (launch_correlate_turned(a, c->stream, c->cfg.corr_path) != 0)
-        return cuda_check(c, cudaGetLastError(), "correlator launch");
+        return launch_failed(c, "correlator launch");
       return DSAX_OK;
     }
   }
   if (launch_correlate(a, fmt, c->stream) != 0)
-    return cuda_check(c, cudaGetLastError(), "correlator launch");
+    return launch_failed(c, "correlator launch");
   return DSAX_OK;
 }
 
@@ -317,7 +323,7 @@ int dsax_corner_turn(dsax_ctx *c, const void *captured, void *out, int out_fmt, 
     if (!aligned16(captured) || !aligned16(out))
       return set_error(c, DSAX_ERR_ARG, "device pointers must be 16-byte aligned");
     if (launch(static_cast<const uint8_t *>(captured), static_cast<uint8_t *>(out)) != 0)
-      return cuda_check(c, cudaGetLastError(), "corner-turn launch");
+      return launch_failed(c, "corner-turn launch");
     return DSAX_OK;
   }
   int rc;
@@ -328,7 +334,7 @@ int dsax_corner_turn(dsax_ctx *c, const void *captured, void *out, int out_fmt, 
   if (e != cudaSuccess) return cuda_check(c, e, "H2D block");
   if (launch(static_cast<const uint8_t *>(c->in_buf.ptr),
              static_cast<uint8_t *>(c->aux[AUX_REORDER_OUT].ptr)) != 0)
-    return cuda_check(c, cudaGetLastError(), "corner-turn launch");
+    return launch_failed(c, "corner-turn launch");
   e = cudaMemcpyAsync(out, c->aux[AUX_REORDER_OUT].ptr, nout, cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_check(c, e, "D2H corner-turned block");
   return dsax_sync(c);

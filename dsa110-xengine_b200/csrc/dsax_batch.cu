@@ -161,7 +161,7 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
     return 0;
   };
   if (!use_graph) {
-    if (enqueue_all() != 0) return cuda_check(c, cudaGetLastError(), "batch launch");
+    if (enqueue_all() != 0) return launch_failed(c, "batch launch");
     return DSAX_OK;
   }
   // (re)capture

@@ -289,7 +289,7 @@ int dsax_beamform(dsax_ctx *c, const void *blk, void *out_u8, void *out_f32, int
     a.out_u8 = static_cast<uint8_t *>(out_u8);
     a.out_f32 = static_cast<float *>(out_f32);
     if (launch_beamform(a, c->num_sms, c->stream) != 0 || !agc_after())
-      return cuda_check(c, cudaGetLastError(), "beamformer launch");
+      return launch_failed(c, "beamformer launch");
     return DSAX_OK;
   }
   int rc;
@@ -303,7 +303,7 @@ int dsax_beamform(dsax_ctx *c, const void *blk, void *out_u8, void *out_f32, int
   a.out_u8 = out_u8 ? static_cast<uint8_t *>(c->aux[AUX_BEAM_U8].ptr) : nullptr;
   a.out_f32 = out_f32 ? static_cast<float *>(c->aux[AUX_BEAM_F32].ptr) : nullptr;
   if (launch_beamform(a, c->num_sms, c->stream) != 0 || !agc_after())
-    return cuda_check(c, cudaGetLastError(), "beamformer launch");
+    return launch_failed(c, "beamformer launch");
   if (out_u8 && (e = cudaMemcpyAsync(out_u8, a.out_u8, nout, cudaMemcpyDeviceToHost, c->stream)) !=
                     cudaSuccess)
     return cuda_check(c, e, "D2H beams");

@@ -77,5 +77,5 @@ extern "C" int dsax_place_packets(dsax_ctx *c, const void *pkts, int npk, int st
       static_cast<const uint8_t *>(pkts), npk, stride, payload, ant_lookup, nlookup, act0, nslots,
       slots_per_seq, static_cast<uint8_t *>(block), static_cast<uint8_t *>(next_block), counts);
   return cudaGetLastError() == cudaSuccess ? DSAX_OK
-                                           : cuda_check(c, cudaGetLastError(), "packet placement");
+                                           : launch_failed(c, "packet placement");
 }

@@ -53,6 +53,9 @@ class DeviceGuard {
 
 int set_error(dsax_ctx *c, int code, const char *fmt, ...);
 int cuda_check(dsax_ctx *c, cudaError_t e, const char *what);
+// The status of a launch that did not happen: never DSAX_OK.  A launcher
+// refuses a shape without a CUDA error, or has read (and so cleared) the error.
+int launch_failed(dsax_ctx *c, const char *what);
 int ensure_buffer(dsax_ctx *c, DevBuf &b, size_t nbytes, const char *what);
 int check_device_error(dsax_ctx *c);
 void release_batch_plan(dsax_ctx *c);

@@ -98,7 +98,7 @@ extern "C" int dsax_extract_ex(dsax_ctx *c, const void *vis, void *out, int orde
       return set_error(c, DSAX_ERR_ARG, "misaligned pointer");
     if (launch_extract(static_cast<const float *>(vis), static_cast<float *>(out), nchan, order,
                        autos, nant, c->stream) != 0)
-      return cuda_check(c, cudaGetLastError(), "extract launch");
+      return launch_failed(c, "extract launch");
     return DSAX_OK;
   }
   int rc;
@@ -114,7 +114,7 @@ extern "C" int dsax_extract_ex(dsax_ctx *c, const void *vis, void *out, int orde
                    cudaSuccess)
     return cuda_check(c, e, "H2D autos");
   if (launch_extract(dv, dout, nchan, order, dauto, nant, c->stream) != 0)
-    return cuda_check(c, cudaGetLastError(), "extract launch");
+    return launch_failed(c, "extract launch");
   if (out && (e = cudaMemcpyAsync(out, dout, nout, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess)
     return cuda_check(c, e, "D2H extract");
   if (autos && (e = cudaMemcpyAsync(autos, dauto, nauto, cudaMemcpyDeviceToHost, c->stream)) !=
@@ -172,7 +172,7 @@ extern "C" int dsax_correlate_extract_ex(dsax_ctx *c, const void *blk, void *out
   float *dauto = !autos ? nullptr
                  : mem == DSAX_MEM_DEVICE ? autos : reinterpret_cast<float *>(base + o_auto);
   if (launch_extract(dv, dout, nchan, order, dauto, nant, c->stream) != 0)
-    return cuda_check(c, cudaGetLastError(), "extract launch");
+    return launch_failed(c, "extract launch");
   if (mem == DSAX_MEM_DEVICE) return DSAX_OK;
   if (out && (e = cudaMemcpyAsync(out, dout, nout, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess)
     return cuda_check(c, e, "D2H extract");

@@ -138,7 +138,7 @@ int dsax_flag(dsax_ctx *c, const dsax_flag_params *p, const float *x, const floa
   if (mem == DSAX_MEM_DEVICE) {
     a.x = x; a.oldspec = oldspec; a.chanmask = chanmask; a.tsmask = tsmask;
     if (!aligned16(x)) return set_error(c, DSAX_ERR_ARG, "filterbank must be 16-byte aligned");
-    if (launch_flag(a, c->stream) != 0) return cuda_check(c, cudaGetLastError(), "flagger launch");
+    if (launch_flag(a, c->stream) != 0) return launch_failed(c, "flagger launch");
     return DSAX_OK;
   }
   const size_t nx = (size_t)B * T * C * 4;
@@ -153,7 +153,7 @@ int dsax_flag(dsax_ctx *c, const dsax_flag_params *p, const float *x, const floa
       (e = cudaMemcpyAsync(dold, oldspec, nbc * 4, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess)
     return cuda_check(c, e, "H2D oldspec");
   a.x = dx; a.oldspec = oldspec ? dold : nullptr; a.chanmask = dm; a.tsmask = dm + nbc;
-  if (launch_flag(a, c->stream) != 0) return cuda_check(c, cudaGetLastError(), "flagger launch");
+  if (launch_flag(a, c->stream) != 0) return launch_failed(c, "flagger launch");
   if ((e = cudaMemcpyAsync(chanmask, dm, nbc, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess ||
       (e = cudaMemcpyAsync(tsmask, dm + nbc, nbt, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess)
     return cuda_check(c, e, "D2H masks");
@@ -318,7 +318,7 @@ int dsax_flag_clean(dsax_ctx *c, dsax_flag_state *st, void *data, uint8_t *chanm
   if (!st->started) {
     // measured only: statistics for the baseline history, no flagging
     a.ts_mean = 1;
-    if (launch_flag_stats(a, c->stream) != 0) return cuda_check(c, cudaGetLastError(), "flag stats");
+    if (launch_flag_stats(a, c->stream) != 0) return launch_failed(c, "flag stats");
     if ((e = cudaMemsetAsync(dcm, 0, bc, c->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(dtm, 0, bt, c->stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(st->hist_spec + (size_t)st->nseen * bc, a.spec, bc * 4,
@@ -330,7 +330,7 @@ int dsax_flag_clean(dsax_ctx *c, dsax_flag_state *st, void *data, uint8_t *chanm
     if (st->nseen >= st->cp.naver) {
       if (launch_flag_baseline(st->hist_spec, st->hist_var, st->cp.naver, B, C, st->spec0,
                                st->var0, c->stream) != 0)
-        return cuda_check(c, cudaGetLastError(), "flag baseline");
+        return launch_failed(c, "flag baseline");
       st->started = 1;
     }
     st->last_flagged = 0;
@@ -347,7 +347,7 @@ int dsax_flag_clean(dsax_ctx *c, dsax_flag_state *st, void *data, uint8_t *chanm
     if ((e = cudaMemcpyAsync(st->tpwr + 2, st->tpwr, 8, cudaMemcpyDeviceToDevice, c->stream)) !=
         cudaSuccess)
       return cuda_check(c, e, "total power");
-    if (launch_flag(a, c->stream) != 0) return cuda_check(c, cudaGetLastError(), "flagger launch");
+    if (launch_flag(a, c->stream) != 0) return launch_failed(c, "flagger launch");
     // after a flagged block its total power is the next comparison (:1401)
     if ((e = cudaMemcpyAsync(st->tpwr, st->tpwr + 1, 8, cudaMemcpyDeviceToDevice, c->stream)) !=
         cudaSuccess)

@@ -192,7 +192,7 @@ int dsax_lf_features(dsax_ctx *c, const float *x, const dsax_flag_params *p, int
   LfScratch s;
   if ((rc = lf_scratch(c, p->nbeam, p->ntime / tds, p->nchan, p->ntime, p->tbin, s)) != DSAX_OK) return rc;
   if (lf_make_features(p, x, tds, s, F, nullptr, c->stream) != 0)
-    return cuda_check(c, cudaGetLastError(), "feature launch");
+    return launch_failed(c, "feature launch");
   return DSAX_OK;
 }
 
@@ -210,8 +210,10 @@ int dsax_lf_train_step(dsax_ctx *c, const float *x, const uint8_t *chanmask, con
   LfNet &net = *c->lf;
   float *acts[5] = {s.F, s.a1, s.a2, s.a3, s.z};
   const int nvalid = B * H * (W - 2 * p->guard);
+  // (no step on features that were not made: it would move the parameters)
+  if (lf_make_features(p, x, tds, s, s.F, nullptr, c->stream) != 0)
+    return launch_failed(c, "feature launch");
   int e = 0;
-  e |= lf_make_features(p, x, tds, s, s.F, nullptr, c->stream);
   e |= lf_labels(chanmask, tsmask, s.L, B, p->ntime, W, tds, p->guard, c->stream);
   e |= lf_prepare_weights(net, c->stream);
   e |= lf_forward(net, acts, B, H, W, c->stream);
@@ -219,8 +221,8 @@ int dsax_lf_train_step(dsax_ctx *c, const float *x, const uint8_t *chanmask, con
   e |= lf_bce(s.z, s.L, s.d4, s.loss, B, H, W, p->guard, pos_weight, 1.0f / (float)nvalid,
               c->stream);
   e |= lf_backward(net, acts, s.d4, s.da, s.db, s.part, B, H, W, c->stream);
-  if (update) e |= lf_adam(net, lr, c->stream);
-  if (e) return cuda_check(c, cudaGetLastError(), "training step launch");
+  if (update && !e) e |= lf_adam(net, lr, c->stream);
+  if (e) return launch_failed(c, "training step launch");
   if (loss) {
     double h = 0.0;
     cudaError_t ce = cudaMemcpyAsync(&h, s.loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
@@ -293,15 +295,16 @@ int dsax_flag_learned(dsax_ctx *c, const float *x, const dsax_flag_params *p, in
   LfPerm perm;
   perm.n = p->nperm;
   for (int k = 0; k < p->nperm; ++k) perm.ch[k] = p->perm[k];
+  if (lf_make_features(p, xd, tds, s, nullptr, fbf, c->stream) != 0)
+    return launch_failed(c, "feature launch");
   int e = 0;
-  e |= lf_make_features(p, xd, tds, s, nullptr, fbf, c->stream);
   if (c->lf_wimg_version != net.version) {   // weight images of the current parameters
     e |= lf_tc_prepare(net, static_cast<uint8_t *>(c->aux[AUX_LF_TCW].ptr), c->stream);
     if (!e) c->lf_wimg_version = net.version;
   }
   e |= lf_tc_forward(net, tb, B, H, W, p->guard, perm, zero_borders, c->num_sms, c->d_err,
                      c->cfg.wait_limit_ns, c->stream);
-  if (e) return cuda_check(c, cudaGetLastError(), "learned flagger launch");
+  if (e) return launch_failed(c, "learned flagger launch");
   if (zero_borders) {
     c->lf_pad_geom[0] = B;
     c->lf_pad_geom[1] = H;

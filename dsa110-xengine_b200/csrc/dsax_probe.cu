@@ -123,7 +123,7 @@ extern "C" int dsax_probe_tensor_peak(dsax_ctx *c, int kind, int reps, double *o
   for (int r = 0; r <= reps && rc == DSAX_OK; ++r) {   // the first launch warms up
     cudaEventRecord(e0, c->stream);
     if (launch() != 0) {
-      rc = cuda_check(c, cudaGetLastError(), "probe launch");
+      rc = launch_failed(c, "probe launch");
       break;
     }
     cudaEventRecord(e1, c->stream);
