@@ -153,12 +153,15 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
     if (cudaEventRecord(c->bev[0], c->stream) != cudaSuccess ||
         cudaStreamWaitEvent(c->bstream, c->bev[0], 0) != cudaSuccess)
       return -2;
-    for (int i = 0; i < nblk; ++i)
-      if (enqueue_block(c, blocks[i], scratch, fb, fs, c->stream, c->bstream) != 0) return -2;
+    int rc2 = 0;
+    for (int i = 0; i < nblk && rc2 == 0; ++i)
+      rc2 = enqueue_block(c, blocks[i], scratch, fb, fs, c->stream, c->bstream);
+    // joined after a refused block too: later work on the context stream
+    // follows what the other chain holds, and a capture ends whole
     if (cudaEventRecord(c->bev[1], c->bstream) != cudaSuccess ||
         cudaStreamWaitEvent(c->stream, c->bev[1], 0) != cudaSuccess)
       return -2;
-    return 0;
+    return rc2;
   };
   if (!use_graph) {
     if (enqueue_all() != 0) return launch_failed(c, "batch launch");
@@ -177,7 +180,11 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
   if (e != cudaSuccess) return cuda_check(c, e, "begin capture");
   const int lrc = enqueue_all();
   e = cudaStreamEndCapture(c->stream, &plan->graph);
-  if (lrc || e != cudaSuccess) return cuda_check(c, e != cudaSuccess ? e : cudaErrorUnknown, "capture");
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // the capture's error is reported here, not left for the next call
+    return cuda_check(c, e, "capture");
+  }
+  if (lrc) return launch_failed(c, "batch launch");
   e = cudaGraphInstantiate(&plan->exec, plan->graph, 0);
   if (e != cudaSuccess) return cuda_check(c, e, "graph instantiate");
   e = cudaGraphLaunch(plan->exec, c->stream);
