@@ -21,6 +21,9 @@ namespace {
 
 struct BatchPlan {
   std::vector<dsax_block_desc> blocks;
+  // the context's scratch that the graph's kernels use: a larger batch in
+  // between moves it
+  const void *scratch = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -136,7 +139,7 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
   float *fs = fb + nfb;
 
   BatchPlan *plan = static_cast<BatchPlan *>(c->batch_plan);
-  bool same = plan && (int)plan->blocks.size() == nblk &&
+  bool same = plan && plan->scratch == scratch && (int)plan->blocks.size() == nblk &&
               memcmp(plan->blocks.data(), blocks, sizeof(dsax_block_desc) * nblk) == 0;
   if (use_graph && same && plan->exec) {
     cudaError_t e = cudaGraphLaunch(plan->exec, c->stream);
@@ -176,6 +179,7 @@ int dsax_run_batch(dsax_ctx *c, const dsax_block_desc *blocks, int nblk, int use
   plan = new BatchPlan();
   c->batch_plan = plan;
   plan->blocks.assign(blocks, blocks + nblk);
+  plan->scratch = scratch;
   cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_check(c, e, "begin capture");
   const int lrc = enqueue_all();
