@@ -1225,8 +1225,8 @@ size_t flag_part_bytes(int nbeam, int ntime, int nchan, int tbin, bool table) {
                : 0;
 }
 
-// The library-wide error word of flagger launches made without a context
-// (dsax_flag_noalloc, the learned-flagger features), one per device.
+// The error word of flagger launches made without a context
+// (dsax_flag_noalloc, which has none to report to), one per device.
 static __device__ int g_flag_err;
 static int *flag_err_word() {
   int dev = 0;

@@ -114,11 +114,15 @@ int lf_scratch(dsax_ctx *c, int B, int H, int W, int T, int tbin, LfScratch &s) 
 
 // Features of a device filterbank: the statistics pass (the plain flagger's
 // staged kernel, also writing the downsampled spectrogram) then the
-// per-beam feature kernel.
-int lf_make_features(const dsax_flag_params *p, const float *x, int tds, const LfScratch &s,
-                     float *F, uint16_t *Fbf, cudaStream_t st) {
+// per-beam feature kernel.  A wait of the pass that runs out is the context's
+// error, as every other one: its CTA leaves its statistics unwritten.
+int lf_make_features(dsax_ctx *c, const dsax_flag_params *p, const float *x, int tds,
+                     const LfScratch &s, float *F, uint16_t *Fbf) {
+  cudaStream_t st = c->stream;
   const int B = p->nbeam, T = p->ntime, C = p->nchan, H = T / tds;
   FlagArgs a{};
+  a.err = c->d_err;
+  a.wait_limit_ns = c->cfg.wait_limit_ns;
   a.x = x;
   a.nbeam = B; a.ntime = T; a.nchan = C;
   a.guard = p->guard; a.filt = p->filt; a.tbin = p->tbin; a.fbin = p->fbin;
@@ -191,7 +195,7 @@ int dsax_lf_features(dsax_ctx *c, const float *x, const dsax_flag_params *p, int
   DeviceGuard g(c->device);
   LfScratch s;
   if ((rc = lf_scratch(c, p->nbeam, p->ntime / tds, p->nchan, p->ntime, p->tbin, s)) != DSAX_OK) return rc;
-  if (lf_make_features(p, x, tds, s, F, nullptr, c->stream) != 0)
+  if (lf_make_features(c, p, x, tds, s, F, nullptr) != 0)
     return launch_failed(c, "feature launch");
   return DSAX_OK;
 }
@@ -211,7 +215,7 @@ int dsax_lf_train_step(dsax_ctx *c, const float *x, const uint8_t *chanmask, con
   float *acts[5] = {s.F, s.a1, s.a2, s.a3, s.z};
   const int nvalid = B * H * (W - 2 * p->guard);
   // (no step on features that were not made: it would move the parameters)
-  if (lf_make_features(p, x, tds, s, s.F, nullptr, c->stream) != 0)
+  if (lf_make_features(c, p, x, tds, s, s.F, nullptr) != 0)
     return launch_failed(c, "feature launch");
   int e = 0;
   e |= lf_labels(chanmask, tsmask, s.L, B, p->ntime, W, tds, p->guard, c->stream);
@@ -295,7 +299,7 @@ int dsax_flag_learned(dsax_ctx *c, const float *x, const dsax_flag_params *p, in
   LfPerm perm;
   perm.n = p->nperm;
   for (int k = 0; k < p->nperm; ++k) perm.ch[k] = p->perm[k];
-  if (lf_make_features(p, xd, tds, s, nullptr, fbf, c->stream) != 0)
+  if (lf_make_features(c, p, xd, tds, s, nullptr, fbf) != 0)
     return launch_failed(c, "feature launch");
   int e = 0;
   if (c->lf_wimg_version != net.version) {   // weight images of the current parameters
