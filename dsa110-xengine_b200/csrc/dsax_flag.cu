@@ -36,6 +36,9 @@ namespace dsax {
 namespace flag {
 constexpr int kStatThreads = 256;
 constexpr int kTargetCtas = 296;      // statistics CTAs below which time is chunked: two per SM
+// Shared memory of a statistics CTA that leaves room for a second one: half of
+// an SM's 228 KB, less the 1 KB that each CTA takes and 6.5 KB of static arrays.
+constexpr size_t kStatSmem = 114 * 1024 - 1024 - 6656;
 constexpr int kMaxChan = 1024;
 constexpr int kApplyThreads = 256;    // apply / time-series CTA
 constexpr int kApplyRows = 256;       // rows per apply CTA
@@ -1280,10 +1283,11 @@ int launch_flag_stats(FlagArgs a, cudaStream_t st) {
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   if (encode_filterbank_map(&map, a, brows) != 0) return -2;
-  // as deep a ring as lets two CTAs share an SM
+  // as deep a ring as lets two CTAs share an SM (20 channels, 256 beams x 512
+  // samples: 47.7 us with one CTA per SM and three boxes, 34.3 with two CTAs)
   size_t sh = 0;
   for (a.ring = flag::kMaxRing; a.ring >= 2; --a.ring)
-    if ((sh = stats_smem(a, es)) <= 112 * 1024 || a.ring == 2) break;
+    if ((sh = stats_smem(a, es)) <= flag::kStatSmem || a.ring == 2) break;
   const dim3 grid(a.nslab * a.nchunk, a.nbeam);
   // full slabs, or the one slab of a 48-channel subband, have their own forms
   const int kind = a.nchan % kFlagSlab == 0 ? 2 : a.nchan == 48 ? 1 : 0;
