@@ -658,12 +658,14 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-// Up to kRankMax values the element of rank k is found by counting instead (one
-// barrier for 16: of the 48 channels' decisions the four-pass select was half).
-constexpr int kRankMax = 128;
+// Few values are ranked by counting instead (two barriers for 16): up to
+// kRankWork comparisons a thread, since they grow with n squared.  A call of 256
+// beams x 64 samples, us, counting / select: 16 channels 28 / 36, 48 32 / 38,
+// 64 36 / 41, 72 (two values a thread of 64) 37 / 34, 96 40 / 37, 128 46 / 36.
+constexpr int kRankWork = 64;
 __device__ __forceinline__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist,
                                                   uint32_t *sel, int gtid, int gsize, int bid) {
-  if (n <= kRankMax) {
+  if (n * ((n + gsize - 1) / gsize) <= kRankWork) {
     for (int i = gtid; i < n; i += gsize) {
       const uint32_t x = ordered_key(v[i]);
       int r = 0;
@@ -762,7 +764,7 @@ __device__ __forceinline__ void window_median(const float *x, float v, float *ou
 __device__ void grp_detrend3(float *sb0, const FlagArgs &a, int gtid, int gsize) {
   const int C = a.nchan, G = a.guard, F = a.filt, n = C - 2 * G;
   const int kf = (F + 1) / 2 - 1;
-  if (F == 21 && n > kRankMax) {   // nFiltSize; few channels: not worth the unrolled code
+  if (F == 21 && n > 128) {   // nFiltSize; few channels: not worth the unrolled code
     for (int id = gtid; id < 3 * n; id += gsize) {
       const int k = id / n, jj = id - k * n;
       float *sb = sb0 + 3 * C * k;
