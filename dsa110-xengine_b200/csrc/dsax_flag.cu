@@ -465,10 +465,12 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
   // warp; the bin's sums combined by the CTA); then the rows beyond the last
   // whole bin: everything but the bins.  (One loop, so that the row code exists
   // once.)
-  // (Split bins go one after the other, each about 2 us of latency and barriers
-  // however short, against 0.4 us per box: from 4 boxes of a single bin to 256
-  // of seven, a warp per bin is no slower.)
-  const bool by_warp = bin1 - bin0 >= kWarps || (TB + brows - 1) / brows <= 2 << (bin1 - bin0);
+  // (Split bins go one after the other, each with its latency and barriers
+  // however short; a warp per bin leaves warps idle.  Up to 2^n boxes in each of
+  // n bins the warp is no slower.  256 beams, us, warp / split: 64 channels, one
+  // bin of 4 boxes 35.8 / 31.9, 256 channels, two of 8 81 / 68, three of 16 130 /
+  // 116; 64 channels, four of 8 48.4 / 48.3, seven of 8 60 / 64.)
+  const bool by_warp = bin1 - bin0 >= kWarps || (TB + brows - 1) / brows <= 1 << (bin1 - bin0);
   const int nbseg = by_warp ? 1 : bin1 - bin0;
   const int ntail = chunk == a.nchunk - 1 ? T - nbins * TB : 0;
   // a short tail goes to a warp that has no bin
