@@ -47,7 +47,7 @@ __global__ void ct_pack_kernel(const uint8_t *__restrict__ in, uint8_t *__restri
 // recv [nsrc][nbl][nt][nc] -> fil[nbl][t0 + t][ch0 + s nc + k] of a
 // filterbank with fil_nt samples and fil_nc channels per row.
 //
-// HBM-bound (every byte read and written once).  A CTA places kCtRows passes
+// HBM-bound (every byte read and written once).  A CTA places kCtPasses passes
 // of rows of one beam; a thread owns one V-byte piece of the row (source s,
 // piece p of its nc bytes) and a row phase, so its source and destination
 // advance by constants and all divisions are done once per thread (one
@@ -57,7 +57,9 @@ __global__ void ct_pack_kernel(const uint8_t *__restrict__ in, uint8_t *__restri
 // loads four in flight (eight 590).  Consecutive threads write
 // consecutive pieces of a filterbank row; the pieces of a source's
 // consecutive rows share lines, which the passes of one CTA find in L1.
-constexpr int kCtThreads = 256, kCtUnroll = 4, kCtRows = 16;
+// (Rows counted from the CTA's first one instead of absolutely: the same loop
+// compiles to another order of the loads, 431 us.)
+constexpr int kCtThreads = 256, kCtUnroll = 4, kCtPasses = 16;
 template <int V>
 __global__ void __launch_bounds__(kCtThreads)
     ct_unpack_kernel(const uint8_t *__restrict__ recv, uint8_t *__restrict__ fil, int nsrc, int nbl,
@@ -71,15 +73,16 @@ __global__ void __launch_bounds__(kCtThreads)
   const int phases = kCtThreads / width;              // rows of a pass
   const int ph = (int)threadIdx.x / width, lane = (int)threadIdx.x - ph * width;
   if (ph >= phases) return;
-  const int r0 = (int)blockIdx.x * kCtRows * phases + ph;
-  const int r1 = min(nt, ((int)blockIdx.x + 1) * kCtRows * phases);
+  const uint32_t r0 = blockIdx.x * (uint32_t)(kCtPasses * phases) + (uint32_t)ph;
+  const uint32_t r1 = min((uint32_t)nt, (blockIdx.x + 1u) * (uint32_t)(kCtPasses * phases));
   for (int q = lane; q < pieces; q += width) {
     const int s = q / pr, p = q - s * pr;
     for (int j = blockIdx.y; j < nbl; j += gridDim.y) {
       const uint8_t *src = recv + (((int64_t)s * nbl + j) * nt + r0) * nc + (int64_t)p * V;
       uint8_t *dst = fil + ((int64_t)j * fil_nt + t0 + r0) * fil_nc + ch0 + (int64_t)q * V;
       const int64_t sstep = (int64_t)phases * nc, dstep = (int64_t)phases * fil_nc;
-      for (int r = r0; r < r1; r += kCtUnroll * phases) {
+#pragma unroll 1
+      for (uint32_t r = r0; r < r1; r += kCtUnroll * phases) {
         W v[kCtUnroll];
 #pragma unroll
         for (int k = 0; k < kCtUnroll; ++k)
@@ -127,8 +130,8 @@ extern "C" int dsax_ct_unpack(dsax_ctx *c, const uint8_t *recv, int nsrc, int nb
   const int V = al % 16 == 0 ? 16 : al % 8 == 0 ? 8 : al % 4 == 0 ? 4 : 1;
   const int pieces = nsrc * (nc / V);
   const int width = pieces < kCtThreads ? pieces : kCtThreads;
-  const int rows = kCtRows * (kCtThreads / width);
-  const dim3 grid((nt + rows - 1) / rows, nbl < 65535 ? nbl : 65535);
+  const int rows = kCtPasses * (kCtThreads / width);
+  const dim3 grid((nt - 1) / rows + 1, nbl < 65535 ? nbl : 65535);
   auto kernel = V == 16 ? ct_unpack_kernel<16> : V == 8 ? ct_unpack_kernel<8>
               : V == 4  ? ct_unpack_kernel<4> : ct_unpack_kernel<1>;
   kernel<<<grid, kCtThreads, 0, c->stream>>>(recv, fil, nsrc, nbl, nt, nc, fil_nt, fil_nc, t0, ch0,
