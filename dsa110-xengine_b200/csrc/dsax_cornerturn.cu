@@ -47,7 +47,7 @@ __global__ void ct_pack_kernel(const uint8_t *__restrict__ in, uint8_t *__restri
 // recv [nsrc][nbl][nt][nc] -> fil[nbl][t0 + t][ch0 + s nc + k] of a
 // filterbank with fil_nt samples and fil_nc channels per row.
 //
-// HBM-bound (every byte read and written once).  A CTA places kCtPasses passes
+// HBM-bound (every byte read and written once).  A CTA places some passes
 // of rows of one beam; a thread owns one V-byte piece of the row (source s,
 // piece p of its nc bytes) and a row phase, so its source and destination
 // advance by constants and all divisions are done once per thread (one
@@ -59,8 +59,10 @@ __global__ void ct_pack_kernel(const uint8_t *__restrict__ in, uint8_t *__restri
 // consecutive rows share lines, which the passes of one CTA find in L1.
 // (Rows counted from the CTA's first one instead of absolutely: the same loop
 // compiles to another order of the loads, 431 us.)
+// A call of few CTAs gives each fewer passes: its time is the chain of one
+// thread's rows (4 x 65,536 rows of 4 bytes: 16 passes 6.1 us, 4 passes 5.4).
 constexpr int kCtThreads = 256, kCtUnroll = 4, kCtPasses = 16;
-template <int V>
+template <int V, int kPasses>
 __global__ void __launch_bounds__(kCtThreads)
     ct_unpack_kernel(const uint8_t *__restrict__ recv, uint8_t *__restrict__ fil, int nsrc, int nbl,
                      int nt, int nc, int fil_nt, int fil_nc, int t0, int ch0, int pieces) {
@@ -73,8 +75,8 @@ __global__ void __launch_bounds__(kCtThreads)
   const int phases = kCtThreads / width;              // rows of a pass
   const int ph = (int)threadIdx.x / width, lane = (int)threadIdx.x - ph * width;
   if (ph >= phases) return;
-  const uint32_t r0 = blockIdx.x * (uint32_t)(kCtPasses * phases) + (uint32_t)ph;
-  const uint32_t r1 = min((uint32_t)nt, (blockIdx.x + 1u) * (uint32_t)(kCtPasses * phases));
+  const uint32_t r0 = blockIdx.x * (uint32_t)(kPasses * phases) + (uint32_t)ph;
+  const uint32_t r1 = min((uint32_t)nt, (blockIdx.x + 1u) * (uint32_t)(kPasses * phases));
   for (int q = lane; q < pieces; q += width) {
     const int s = q / pr, p = q - s * pr;
     for (int j = blockIdx.y; j < nbl; j += gridDim.y) {
@@ -130,10 +132,16 @@ extern "C" int dsax_ct_unpack(dsax_ctx *c, const uint8_t *recv, int nsrc, int nb
   const int V = al % 16 == 0 ? 16 : al % 8 == 0 ? 8 : al % 4 == 0 ? 4 : 1;
   const int pieces = nsrc * (nc / V);
   const int width = pieces < kCtThreads ? pieces : kCtThreads;
-  const int rows = kCtPasses * (kCtThreads / width);
-  const dim3 grid((nt - 1) / rows + 1, nbl < 65535 ? nbl : 65535);
-  auto kernel = V == 16 ? ct_unpack_kernel<16> : V == 8 ? ct_unpack_kernel<8>
-              : V == 4  ? ct_unpack_kernel<4> : ct_unpack_kernel<1>;
+  // (two CTAs per SM, or fewer passes)
+  const int phases = kCtThreads / width;
+  auto blocks = [&](int passes) { return (nt - 1) / (passes * phases) + 1; };
+  const int passes = (int64_t)blocks(kCtPasses) * nbl < 2 * c->num_sms ? kCtUnroll : kCtPasses;
+  const dim3 grid(blocks(passes), nbl < 65535 ? nbl : 65535);
+  const bool few = passes != kCtPasses;
+  auto kernel = V == 16  ? (few ? ct_unpack_kernel<16, kCtUnroll> : ct_unpack_kernel<16, kCtPasses>)
+                : V == 8 ? (few ? ct_unpack_kernel<8, kCtUnroll> : ct_unpack_kernel<8, kCtPasses>)
+                : V == 4 ? (few ? ct_unpack_kernel<4, kCtUnroll> : ct_unpack_kernel<4, kCtPasses>)
+                         : (few ? ct_unpack_kernel<1, kCtUnroll> : ct_unpack_kernel<1, kCtPasses>);
   kernel<<<grid, kCtThreads, 0, c->stream>>>(recv, fil, nsrc, nbl, nt, nc, fil_nt, fil_nc, t0, ch0,
                                              pieces);
   return cuda_check(c, cudaGetLastError(), "corner-turn unpack");
