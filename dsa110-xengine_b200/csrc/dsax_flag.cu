@@ -51,17 +51,6 @@ constexpr int kDecThreads = 256;
 // ---------------------------------------------------------------- elements
 // Four consecutive channels of one row: FP32 (16 bytes) or uint8 (4 bytes).
 template <typename E>
-__device__ __forceinline__ void ld4(const void *p, float (&v)[4]) {
-  if constexpr (std::is_same<E, float>::value) {
-    const float4 t = *reinterpret_cast<const float4 *>(p);
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-  } else {
-    const uint32_t w = *reinterpret_cast<const uint32_t *>(p);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = (float)((w >> (8 * j)) & 255u);
-  }
-}
-template <typename E>
 __device__ __forceinline__ void st4(void *p, const float (&v)[4]) {
   if constexpr (std::is_same<E, float>::value) {
     *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -148,9 +137,12 @@ constexpr int kPartFields = 5;   // per channel of a chunk: sum, squares, max, b
 }  // namespace flag
 
 // kPix: also forms the downsampled spectrogram.  kG: the slab's 4-channel
-// groups where they are known when compiling (12, the 48 channel groups of a
-// subband; 32, a full slab), so that row and table strides are constants: a
-// third of the instructions of the general form (0).
+// groups where they are known when compiling, so that row and table strides are
+// constants: 32, a full slab, and 12, the 48 channel groups that the beamformer
+// makes of the library's default subband (384 channels).  At 48 channels, us,
+// constant / general form (0): masks of 256 x 4,096 FP32 107.6 / 114.7, cleaning
+// 64 x 16,384 uint8 113 / 123, learned-flagger features of 256 x 4,096 104 / 124.
+// The pixel form has no full slab (it is used up to 64 channels).
 template <typename E, bool kPix, int kG>
 __global__ void __launch_bounds__(flag::kStatThreads, 2)
     flag_stats_kernel(const __grid_constant__ CUtensorMap tmap, FlagArgs a) {
@@ -1294,12 +1286,11 @@ int launch_flag_stats(FlagArgs a, cudaStream_t st) {
     if ((sh = stats_smem(a, es)) <= flag::kStatSmem || a.ring == 2) break;
   const dim3 grid(a.nslab * a.nchunk, a.nbeam);
   // full slabs, or the one slab of a 48-channel subband, have their own forms
-  const int kind = a.nchan % kFlagSlab == 0 ? 2 : a.nchan == 48 ? 1 : 0;
+  const int kind = a.nchan == 48 ? 1 : a.nchan % kFlagSlab == 0 && !a.pix_sum ? 2 : 0;
   void (*const kernels[3][3])(const CUtensorMap, FlagArgs) = {
       {flag_stats_kernel<uint8_t, false, 0>, flag_stats_kernel<uint8_t, false, 12>,
        flag_stats_kernel<uint8_t, false, 32>},
-      {flag_stats_kernel<float, true, 0>, flag_stats_kernel<float, true, 12>,
-       flag_stats_kernel<float, true, 32>},
+      {flag_stats_kernel<float, true, 0>, flag_stats_kernel<float, true, 12>, nullptr},
       {flag_stats_kernel<float, false, 0>, flag_stats_kernel<float, false, 12>,
        flag_stats_kernel<float, false, 32>}};
   const int row = u8 ? 0 : a.pix_sum ? 1 : 2;
