@@ -614,7 +614,8 @@ __global__ void __launch_bounds__(flag::kStatThreads, 2)
     a.spec[o] = (float)mean;
     a.var[o] = (float)var;
     a.maxs[o] = a.parity ? (float)mean : (float)tot[2];
-    a.pp[o] = nbins > 0 ? (float)(bmax * inv_tb - bmin * inv_tb) : 0.0f;
+    // (both products rounded: fused into one the difference of equal bins is not 0)
+    a.pp[o] = nbins > 0 ? (float)(__dmul_rn(bmax, inv_tb) - __dmul_rn(bmin, inv_tb)) : 0.0f;
   }
   if (!a.decide) return;
   // The last slab CTA of the beam makes its channel decisions, and the last
