@@ -730,8 +730,8 @@ __device__ __noinline__ float grp_select_call(const float *v, int n, int k, uint
 // One window of channflag's detrend: v - lower median of x[0..kF), the median
 // by rank counting with ties by index, in registers (a thread per window;
 // with a thread per window element and shared loads it was 70 us of the 1,024
-// channels' decisions).  Nothing is written where no element has the rank
-// (NaN data).
+// channels' decisions).  Nothing is written where no element has the rank: the
+// window is mostly NaN, and its caller's NaN stays, which no test flags.
 template <int kF>
 __device__ __forceinline__ void window_median(const float *x, float v, float *out) {
   float e[kF];
@@ -821,8 +821,10 @@ __device__ void flag_decide_beam(const FlagArgs &a, int b, uint8_t *smem) {
   const int g = warp >> 1, gsize = 64, gtid = tid - 64 * g, bid = 1 + g;
   float *sb = dsh + g * 3 * C, *corr = sb + C, *tm = corr + C;
   const float *src = g == 0 ? a.spec : g == 1 ? a.var : g == 2 ? a.maxs : a.pp;
-  for (int c = gtid; c < C; c += gsize)
+  for (int c = gtid; c < C; c += gsize) {
     sb[c] = src[b * C + c] - ((g == 0 && a.oldspec) ? a.oldspec[b * C + c] : 0.0f);
+    corr[c] = NAN;   // what a window without a median leaves
+  }
   __syncthreads();
   // the three detrends by the whole CTA, then a test per group
   grp_detrend3(dsh, a, tid, flag::kStatThreads);
@@ -1375,6 +1377,7 @@ __global__ void __launch_bounds__(2 * flag::kDecThreads) lf_stat_features_kernel
     const int k = i / C, c = i - k * C;
     const float *src = k == 0 ? a.spec : k == 1 ? a.var : k == 2 ? a.maxs : a.pp;
     dsh[3 * C * k + c] = src[b * C + c];
+    dsh[3 * C * k + C + c] = NAN;   // what a window without a median leaves
     z[i] = 0.0f;
   }
   for (int i = tid; i < a.ts_base; i += blockDim.x) zt[i] = tsb[i];
