@@ -111,16 +111,17 @@ __device__ void flag_total_power(const FlagArgs &a);
 // barriers and a partly idle row reduction each: 82 against 63 us for
 // [256][4096][48] FP32, of which some 26 are what a call costs at any length;
 // loads straight into registers: 94.  Scaled uint8 [64][16384][1024]: 1,138
-// against 700.)  What bounds it: the loop runs near the HBM rate for FP32; for
-// uint8 the 128-byte slab rows in and out (about 3.6 TB/s), in 1.7 waves of
-// CTAs.
+// against 700.)  What bounds it: instructions and waits, not HBM (FP32 [256]
+// [4096][48]: DRAM at 40 %, issue slots 50 %).  Scaled uint8 [64][16384][1024]
+// reads and writes 2.15 GB at 3.07 TB/s, issue slots 53 %, in 1.73 waves of CTAs
+// (a single wave of 256 CTAs: 230 us).
 //
 // Sums are FP64 for FP32 data and exact integers for uint8: 32 bits within a
 // range of rows (a lane's share of a bin or of the tail is at most 49,152 rows
 // of an accepted block, so the 255^2 products stay below 2^32; flag_shape_ok),
 // 64 bits for the squares from there on, since a lane may have several bins.
-// Four rows of uint8 are transposed to words of one
-// channel, whose sum and sum of squares are one dp4a each.  A lane's sums are
+// Four rows of uint8 are transposed to words of one channel, whose sum and sum
+// of squares are one dp4a each.  A lane's sums are
 // combined with the other row phases' in a fixed order, and the chunks' by the
 // chunk CTA that finishes last, in chunk order, so results do not depend on
 // scheduling.  With a scaley baseline each value is normalised as it is read
@@ -653,23 +654,25 @@ __device__ __forceinline__ uint32_t ordered_key(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
-// Few values are ranked by counting instead (two barriers for 16): up to
-// kRankWork comparisons a thread, since they grow with n squared.  A call of 256
-// beams x 64 samples, us, counting / select: 16 channels 28 / 36, 48 32 / 38,
-// 64 36 / 41, 72 (two values a thread of 64) 37 / 34, 96 40 / 37, 128 46 / 36.
-constexpr int kRankWork = 64;
+// Few values are ranked by counting instead (two barriers for 16), one a thread:
+// a second one doubles the loop.  A call of 256 beams x 64 samples, us, counting /
+// select by 64 threads: 16 channels 28 / 36, 48 32 / 38, 64 36 / 41, 72 37 / 34, 96
+// 40 / 37, 128 46 / 36; of 4,096 samples x 8 channels with 96 in the time series'
+// base, by 256 threads, 16 beams 35.0 / 36.2, 256 beams 69.1 / 68.7, with 128 36.0 /
+// 36.2 and 71.5 / 68.7.
+constexpr int kRankMax = 96;
 __device__ __forceinline__ float grp_radix_select(const float *v, int n, int k, uint32_t *hist,
                                                   uint32_t *sel, int gtid, int gsize, int bid) {
-  if (n * ((n + gsize - 1) / gsize) <= kRankWork) {
-    for (int i = gtid; i < n; i += gsize) {
-      const uint32_t x = ordered_key(v[i]);
+  if (n <= gsize && n <= kRankMax) {
+    if (gtid < n) {
+      const uint32_t x = ordered_key(v[gtid]);
       int r = 0;
 #pragma unroll 4
       for (int q = 0; q < n; ++q) {
         const uint32_t y = ordered_key(v[q]);
-        r += y < x || (y == x && q < i);
+        r += y < x || (y == x && q < gtid);
       }
-      if (r == k) sel[0] = __float_as_uint(v[i]);
+      if (r == k) sel[0] = __float_as_uint(v[gtid]);
     }
     named_bar(bid, gsize);
     const float out = __uint_as_float(sel[0]);
