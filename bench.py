@@ -44,7 +44,9 @@ REALTIME_S = 0.134217728          # one block of 4096 x 32.768 us samples
 BLOCK_IN = 198_180_864
 VIS_OUT = 51_118_080
 ALG_OPS = 8 * 2080 * 4 * 768 * 2048   # one complex MAC = 8 integer ops
-MMA_OPS = 2 * 128 * 256 * 4096 * 768  # executed tensor-core ops
+# executed tensor-core ops: three 128 x 128 products per frequency (the fused
+# kernel of corr_path 1 has four)
+MMA_OPS = 2 * 3 * 128 * 128 * 2048 * 768
 METRIC = "X-engine blocks/s (full 198 MB block, bit-exact correlate)"
 UNIT = "blocks/s"
 
@@ -614,7 +616,7 @@ def main():
     ap.add_argument("--corr-path", type=int, default=0,
                     help="0 default (=4), 1 fused kernel, 2 REORDER-layout corner turn, "
                          "3 channel-major corner turn + directly fed correlator, "
-                         "4 the same, bulk-copy fed, 5 as 4 with 16 unpack warps, "
+                         "4 corner turn to frequency streams, 5 as 3 but bulk-copy fed, 16 unpack warps, "
                          "6 captured block read directly by 4-CTA clusters, 7 as 6 with 16 unpack warps")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
@@ -807,6 +809,7 @@ def main():
         dom = max(kernel_ms, key=kernel_ms.get)
         corr_ms = [v for k, v in kernel_ms.items() if k.startswith("corr")][0]
         dom_ms = kernel_ms[dom]
+        mma_ops = MMA_OPS * 4 // 3 if cfg.corr_path == 1 else MMA_OPS
         reo_bytes = 2048 * 768 * 64 * 2
         if dom.startswith("reorder"):
             alg = BLOCK_IN + reo_bytes
@@ -849,12 +852,12 @@ def main():
                          "peak_kind": f"{peak_kind} (HBM copy bandwidth)",
                          "alg_bytes_per_launch": alg,
                          "int8_alg_tops": ALG_OPS / (corr_ms * 1e-3) / 1e12,
-                         "int8_mma_tops": MMA_OPS / (corr_ms * 1e-3) / 1e12,
+                         "int8_mma_tops": mma_ops / (corr_ms * 1e-3) / 1e12,
                          "int8_peak_probe_tops": probes.get("int8_tops"),
                          "int8_alg_frac_of_probe": (ALG_OPS / (corr_ms * 1e-3) / 1e12 /
                                                     probes["int8_tops"]
                                                     if probes.get("int8_tops") else None),
-                         "int8_mma_frac_of_probe": (MMA_OPS / (corr_ms * 1e-3) / 1e12 /
+                         "int8_mma_frac_of_probe": (mma_ops / (corr_ms * 1e-3) / 1e12 /
                                                     probes["int8_tops"]
                                                     if probes.get("int8_tops") else None)},
             "tensor_peaks_probe": dict(probes, how="dsax_probe_tensor_peak: every SM issues "

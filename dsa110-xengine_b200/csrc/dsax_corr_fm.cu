@@ -20,10 +20,13 @@
 // 4-11, two per TMEM lane quarter; warp 12 issues the MMAs; warp 13 the TMA
 // boxes.
 //
-// What bounds it: shared memory.  A stage moves 1,152 128-byte wavefronts
-// (640 of operand reads, 256 of operand stores, 256 of the raw stage in and
-// out) against 768 cycles of MMAs: 56 us for the full block's 96 stages of a
-// CTA; measured 62.  (One CTA per channel with the epilogue between channels:
+// What bounds it: no one unit.  For the full block the MMAs alone take 46 us, the
+// boxes alone 41, everything but the MMAs 47; together 62-65, with the tensor
+// pipe active 69 % of the busy SMs' cycles and shared memory at 66 % of the L1's
+// peak.  (A stage of 768 MMA cycles counts 640 wavefronts of operand reads and
+// 508 of the unpack and the epilogue; the two together are more than the
+// stage's 1,109 cycles, so they do not share one port.)  What is left is how
+// well the roles' waits overlap.  (One CTA per channel with the epilogue between channels:
 // 76.)  Stages of 64 packets 77 us, of 256 73 (half the ring); loads straight
 // into registers instead of boxes 66.  The loops that one thread runs per
 // stage (boxes, MMAs) keep ring positions as counters: with a division by the

@@ -5,7 +5,7 @@
 // each block's H2D copy, promote, xgpuCudaXengine and matrix copy-out
 // before it reads the next (src/dsaX_xgpu.cu:300-357).  Here block i+1's
 // corner turn (HBM-bound) runs on a side stream while block i is correlated
-// (bound by shared memory, with HBM bandwidth to spare), and in host mode
+// (which leaves HBM bandwidth to spare), and in host mode
 // the PCIe copies in and out overlap both.  The fused paths (corr_path 6,
 // 7) have no corner turn: only the copies overlap the correlations.  Buffers are double-buffered and
 // every reuse waits on the event of the stage that last read the buffer.

@@ -436,10 +436,11 @@ __device__ __forceinline__ uint32_t x16_lo(uint32_t w) { return (w << 4) & 0xF0F
 __device__ __forceinline__ uint32_t x16_hi(uint32_t w) { return w & 0xF0F0F0F0u; }
 
 // The sums of products of the 16-fold operands are 256 times the
-// visibilities: at most 2^31 for 65,536 packets, reached only by the real
-// part of an autocorrelation of -8 - 8i throughout, which wraps to the
-// lowest int32 (no other sum can reach it); everything else is exact in
-// FP32 (multiples of 256 below 2^31).
+// visibilities: at most 2^31 for 65,536 packets, reached by the real part of
+// every pair of inputs that both stay at -8 - 8i, which wraps to the lowest
+// int32.  No sum reaches -2^31 (the most negative real part is -112 * 256 *
+// 65,536), so that pattern is unambiguous; everything else is exact in FP32
+// (multiples of 256 below 2^31).
 __device__ __forceinline__ float vis_re(uint32_t v) {
   return v == 0x80000000u ? 8388608.0f : (float)(int32_t)v * 0.00390625f;
 }

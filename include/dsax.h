@@ -248,7 +248,7 @@ int dsax_reorder(dsax_ctx *ctx, const void *captured, void *reordered, int mem);
 
 /* Corner turn of a captured block into out_fmt = DSAX_FMT_REORDERED (as
  * dsax_reorder) or DSAX_FMT_CHANMAJOR (one contiguous stream per channel,
- * the layout the default correlator path reads). */
+ * the layout that corr_path 3 and 5 correlate from). */
 int dsax_corner_turn(dsax_ctx *ctx, const void *captured, void *out, int out_fmt, int mem);
 int dsax_correlate_fmt(dsax_ctx *ctx, int fmt, const void *in, void *vis, int mem,
                        int accumulate);
